@@ -148,7 +148,12 @@ typedef struct jq_tune {
                             and not run; the state buffers then hold the
                             state before them (jq_sweep applies the passes
                             the plan keeps), and other out types fail with
-                            JQ_EINVAL.                                         */
+                            JQ_EINVAL.  A plan of one-wire unitaries and
+                            affine permutations only (default tile sizes,
+                            jit 0, 9 qubits or more) moves no amplitude for
+                            any permutation: its state buffers hold the
+                            amplitudes at linearly mapped indices, up to
+                            signs, for jq_adjoint of the same plan.            */
 } jq_tune;
 
 /* Plan summary. */

@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/jqsim.h"
+#include "frame.h"
 
 namespace jq {
 
@@ -150,6 +151,8 @@ struct DeviceTables {
   int32_t* perm_pool = nullptr;
   double* obs_pool = nullptr;     // dense observables, complex128
   void* obs_desc = nullptr;       // DevObs array
+  FrameDev frame;                 // frame plan (plan->frame.on)
+  void* frame_obs = nullptr;      // DevObs array over physical bits
   void* jit = nullptr;            // JitModule of the forward schedule (or nullptr)
   bool jit_tried = false;
   int jit_rc = 0;                 // nonzero: the required specialisation failed
@@ -184,6 +187,8 @@ struct jq_plan {
   std::vector<int32_t> perm_pool;
   std::vector<jq::DevObs> obs;
   std::vector<double> obs_pool;
+  jq::FramePlan frame;               // expectation-value plans of one-wire unitaries and affine permutations
+  std::vector<jq::DevObs> frame_obs; // their Z words over physical bits
   jq::Schedule fwd, adj, bwd;  // bwd: one block per pass (the unfused order; diagnostics)
   int64_t bmat_stride = 0;     // run-dtype complex elements per instance
   int64_t grad_stride = 0;     // complex128 elements per instance

@@ -2105,7 +2105,7 @@ int device_tables(const jq_plan* cplan, const DeviceTables** out) {
   if ((rc = upload(plan->fwd.rops, &t.fwd_rops))) return rc;
   if ((rc = upload(plan->bwd.steps, &t.bwd_steps))) return rc;
   if ((rc = upload(plan->bwd.rops, &t.bwd_rops))) return rc;
-  if (plan->jit && jit_available()) {
+  if (plan->jit && !plan->frame.on && jit_available()) {
     JitModule* jm = new JitModule();
     if ((rc = jit_build(plan, plan->fwd, jm)) == JQ_OK) {
       t.jit = jm;
@@ -2122,6 +2122,12 @@ int device_tables(const jq_plan* cplan, const DeviceTables** out) {
   } else if (plan->jit_required) {
     t.jit_rc = JQ_EUNSUPPORTED;
     t.jit_err = "jq_tune.jit = 1 but NVRTC or the CUDA driver entry points are not available";
+  }
+  if (plan->frame.on) {
+    if ((rc = frame_upload(plan, &t.frame))) return rc;
+    DevObs* fo = nullptr;
+    if ((rc = upload(plan->frame_obs, &fo))) return rc;
+    t.frame_obs = fo;
   }
   t.jit_tried = true;
   plan->dev.push_back(t);
@@ -2224,6 +2230,7 @@ int run_passes(const jq_plan* plan, const Schedule& sch, const TileOp* dops, con
                const RegOp* drops, const DeviceTables* T, typename CplxT<R>::T* state, int batch,
                const typename CplxT<R>::T* bmat, size_t p0, size_t p1, cudaStream_t st,
                const JitModule* jm = nullptr) {
+  if (plan->frame.on) return frame_forward(plan, T->frame, state, batch, bmat, sm_count(), st);
   constexpr int RB = 4;
   for (size_t p = p0; p < p1; ++p) {
     const PassDesc& pd = sch.passes[p];
@@ -2262,6 +2269,8 @@ int prep(const jq_plan* plan, const DeviceTables* T, int batch, const double* an
          typename CplxT<R>::T* bmat, double2* scratch, cudaStream_t st) {
   const int nbk = static_cast<int>(plan->blocks.size());
   if (nbk == 0) return JQ_OK;
+  if (plan->frame.on)
+    return frame_prep(plan, T->frame, T->blocks, T->prims, T->ops, T->const_pool, batch, angles, bmat, st);
   const int64_t work = static_cast<int64_t>(nbk) * batch;
   const int threads = 128;
   const int grid = static_cast<int>((work + threads - 1) / threads);
@@ -2296,20 +2305,21 @@ int measure(const jq_plan* plan, const DeviceTables* T, int batch, int out_type,
     if (n_obs == 0) return JQ_OK;
     double* o = static_cast<double*>(out);
     JQ_CUDA(cudaMemsetAsync(o, 0, sizeof(double) * n_obs * batch, st));
-    const DevObs* od = static_cast<const DevObs*>(T->obs_desc);
+    const std::vector<DevObs>& pobs = plan->frame.on ? plan->frame_obs : plan->obs;
+    const DevObs* od = static_cast<const DevObs*>(plan->frame.on ? T->frame_obs : T->obs_desc);
     const double2* pool = reinterpret_cast<const double2*>(T->obs_pool);
     // Pauli observables in chunks; dense ones one launch each
     int i = 0;
     while (i < n_obs) {
-      if (plan->obs[i].kind == JQ_OBS_PAULI) {
+      if (pobs[i].kind == JQ_OBS_PAULI) {
         // runs of Pauli words that are all Z strings (or all not), kObsChunk at
         // most (kZMax for the one-read Z-string kernel, statevectors of n >= 9)
-        const bool zdiag = plan->obs[i].x_mask == 0 && (plan->obs[i].z_mask >> 35) == 0;
+        const bool zdiag = pobs[i].x_mask == 0 && (pobs[i].z_mask >> 35) == 0;
         const bool zstr = zdiag && !dm && n >= 9;
         const int chunk = zstr ? kZMax : kObsChunk;
         int j = i;
-        while (j < n_obs && j - i < chunk && plan->obs[j].kind == JQ_OBS_PAULI &&
-               (plan->obs[j].x_mask == 0 && (plan->obs[j].z_mask >> 35) == 0) == zdiag)
+        while (j < n_obs && j - i < chunk && pobs[j].kind == JQ_OBS_PAULI &&
+               (pobs[j].x_mask == 0 && (pobs[j].z_mask >> 35) == 0) == zdiag)
           ++j;
         const int gx = std::max(1, std::min<int>(static_cast<int>((dim + threads - 1) / threads),
                                                  std::max(1, 4 * sm_count() / std::max(batch, 1))));
@@ -2329,7 +2339,7 @@ int measure(const jq_plan* plan, const DeviceTables* T, int batch, int out_type,
         }
         i = j;
       } else {
-        const int64_t groups = dim >> plan->obs[i].k;
+        const int64_t groups = dim >> pobs[i].k;
         const int gx = std::max(1, std::min<int>(static_cast<int>((groups + threads - 1) / threads),
                                                  std::max(1, 4 * sm_count() / std::max(batch, 1))));
         for (int b0 = 0; b0 < batch; b0 += kMaxGridY) {
@@ -2411,7 +2421,8 @@ int seed_sv(const jq_plan* plan, const DeviceTables* T, int batch, int out_type,
   switch (out_type) {
     case JQ_OUT_EXPVAL:
       k_seed_expval_sv<R><<<grid_for(dim * batch, threads), threads, 0, st>>>(
-          psi, lam, plan->n_qubits, batch, static_cast<const DevObs*>(T->obs_desc), static_cast<int>(plan->obs.size()),
+          psi, lam, plan->n_qubits, batch, static_cast<const DevObs*>(plan->frame.on ? T->frame_obs : T->obs_desc),
+          static_cast<int>(plan->obs.size()),
           reinterpret_cast<const double2*>(T->obs_pool), ct);
       break;
     case JQ_OUT_STATE:
@@ -2506,10 +2517,26 @@ int adjoint_impl(const jq_plan* plan, int batch, const double* angles, const voi
   double2* gacc = reinterpret_cast<double2*>(w + L.gacc);
   const int64_t elems = plan->state_elems;
   if ((rc = prep<R>(plan, T, batch, angles, mats, bmat, scratch, st))) return rc;
-  JQ_CUDA(cudaMemcpyAsync(psi, state, sizeof(C) * elems * batch, cudaMemcpyDeviceToDevice, st));
-  if ((rc = seed_sv<R>(plan, T, batch, out_type, psi, ct, ct_state, lam, st))) return rc;
   const bool want_grad = (grad_angles || grad_mats) && plan->grad_stride > 0;
   if (want_grad) JQ_CUDA(cudaMemsetAsync(gacc, 0, 16 * static_cast<size_t>(plan->grad_stride) * batch, st));
+  if (plan->frame.on) {
+    // the first pass reads `state` and writes psi, so no copy precedes it
+    if ((rc = seed_sv<R>(plan, T, batch, out_type, static_cast<const C*>(state), ct, ct_state, lam, st))) return rc;
+    const int64_t gs = 2 * plan->grad_stride;
+    double* ga = reinterpret_cast<double*>(gacc);
+    if ((rc = frame_adjoint(plan, T->frame, state, psi, lam, batch, bmat, want_grad ? ga : nullptr, gs, sm_count(), st)))
+      return rc;
+    if (grad_init) JQ_CUDA(cudaMemcpyAsync(grad_init, lam, sizeof(C) * elems * batch, cudaMemcpyDeviceToDevice, st));
+    if (grad_angles && plan->n_angles > 0)
+      JQ_CUDA(cudaMemsetAsync(grad_angles, 0, sizeof(double) * plan->n_angles * batch, st));
+    if (grad_mats && plan->n_mats > 0)
+      JQ_CUDA(cudaMemsetAsync(grad_mats, 0, 16 * static_cast<size_t>(plan->n_mats) * batch, st));
+    if (!want_grad) return JQ_OK;
+    return frame_chain(plan, T->frame, T->blocks, T->prims, T->ops, T->const_pool, batch, angles, bmat, ga, gs,
+                       grad_angles, st);
+  }
+  JQ_CUDA(cudaMemcpyAsync(psi, state, sizeof(C) * elems * batch, cudaMemcpyDeviceToDevice, st));
+  if ((rc = seed_sv<R>(plan, T, batch, out_type, psi, ct, ct_state, lam, st))) return rc;
   // Specialised adjoint: the forward schedule's passes in reverse, each one
   // kernel holding both tiles (psi and lam) in shared memory.
   const JitModule* jm = static_cast<const JitModule*>(T->jit);
@@ -2786,6 +2813,8 @@ int jq_plan_free(jq_plan* plan) {
     cudaFree(t.ops); cudaFree(t.prims); cudaFree(t.blocks); cudaFree(t.fwd_ops); cudaFree(t.adj_ops);
     cudaFree(t.bwd_ops); cudaFree(t.fwd_steps); cudaFree(t.fwd_rops); cudaFree(t.bwd_steps); cudaFree(t.bwd_rops);
     cudaFree(t.const_pool);
+    frame_free(&t.frame);
+    cudaFree(t.frame_obs);
     if (t.jit) {
       jit_free(static_cast<JitModule*>(t.jit));
       delete static_cast<JitModule*>(t.jit);
@@ -2818,6 +2847,14 @@ int jq_plan_get_info(const jq_plan* plan, jq_plan_info* info) {
   for (const Step& st : plan->fwd.steps) {
     if (st.kind == 0) ++info->n_stages_fwd;
     else ++info->n_smem_ops_fwd;
+  }
+  if (plan->frame.on) {
+    const FramePlan& f = plan->frame;
+    info->n_passes_fwd = info->n_passes_adj = static_cast<int32_t>(f.passes.size());
+    info->n_tile_ops_fwd = static_cast<int32_t>(f.gates.size());
+    info->n_stages_fwd = static_cast<int32_t>(f.stages.size());
+    info->n_smem_ops_fwd = 0;
+    if (!f.passes.empty()) info->tile_bits_fwd = info->tile_bits_adj = f.passes[0].t;
   }
   return JQ_OK;
 }

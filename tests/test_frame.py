@@ -1,0 +1,141 @@
+"""Expectation-value plans of one-wire unitaries and affine permutations run in
+a moving frame (csrc/frame.h).  Values and gradients against the CPU oracle,
+which runs every gate: states of one tile (9 to 12 bits), the first sizes with
+several tiles, odd and batched ones.
+
+Tolerances, set before the first run, are those of the other parity tests:
+1e-10 (complex128) and 1e-5 (complex64), absolute, times the weight of the
+cotangents.
+"""
+import numpy as np
+import pytest
+import torch
+
+import jaqsi_b200 as jq
+from jaqsi_b200 import _lib as L
+from jaqsi_b200 import simulation as sim
+from oracle import sim_np as O
+from tests.helpers import obs_records, to_records
+
+pytestmark = pytest.mark.gpu
+TOL = {torch.complex64: 1e-5, torch.complex128: 1e-10}
+
+
+def _circuit(n, seed, n_gates):
+    """Random rotations, fused constants, X, CX, SWAP; the last gates rotate."""
+
+    def f(p):
+        rng = np.random.default_rng(seed)
+        k = 0
+        for i in range(n_gates):
+            w, v = (int(x) for x in rng.choice(n, 2, replace=False))
+            kind = int(rng.integers(10)) if i < n_gates - n else 3
+            if kind == 0:
+                jq.PauliX(wires=w)
+            elif kind == 1:
+                jq.SWAP(wires=[w, v])
+            elif kind == 2:
+                jq.H(wires=w)
+                jq.S(wires=w)
+            elif kind == 3:
+                jq.Rot(p[k], p[k + 1], p[k + 2], wires=w)
+                k += 3
+            elif kind == 4:
+                jq.RZ(p[k], wires=w)  # a diagonal block
+                k += 1
+            elif kind == 5:
+                jq.RX(p[k], wires=w)
+                jq.PauliRot(p[k + 1], "Y", wires=[w])
+                k += 2
+            else:
+                jq.CX(wires=[w, v])
+        return k
+
+    return f
+
+
+def _plan(script, args, obs, n, dtype):
+    lw = sim.lower_tape(script.record(*args), n)
+    specs, okey = sim._lower_obs(obs, n)
+    return sim.get_plan(lw, specs, okey, n, L.JQ_STATEVECTOR, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("n,gates", [(9, 60), (10, 1), (11, 120), (12, 90), (13, 70), (14, 60), (17, 60)])
+def test_frame_values_and_gradients(n, gates, dtype):
+    body = _circuit(n, 10 * n + gates, gates)
+    rng = np.random.default_rng(n)
+    base = rng.uniform(0, 2 * np.pi, 3 * gates + 3)
+    # exact quarter turns: the rotation's pivot and zero entries
+    base[::5] = rng.integers(0, 5, base[::5].size) * (np.pi / 2)
+    obs = [jq.PauliZ(0), jq.PauliZ(n - 1), jq.build_parity_observable([1, 4]),
+           jq.build_parity_observable([0, 2, 5, 7, n - 1])]
+    ct = rng.normal(size=len(obs))
+    script = jq.Script(lambda p: body(p) and None, n_qubits=n)
+    params = torch.tensor(base, requires_grad=True)
+    ev = script.execute("expval", obs, args=(params,), dtype=dtype)
+    (ev.to(torch.float64) @ torch.tensor(ct, device=ev.device)).backward()
+    recs = to_records(script.record(torch.tensor(base)))
+    ev_ref, g_ref = O.adjoint_grad(recs, n, obs_records(obs), ct=ct)
+    np.testing.assert_allclose(ev.detach().cpu().numpy(), ev_ref, atol=TOL[dtype], rtol=0)
+    np.testing.assert_allclose(params.grad.numpy()[: len(g_ref)], g_ref, atol=TOL[dtype] * max(1.0, np.abs(ct).sum()),
+                               rtol=0)
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("n,batch", [(9, 3), (12, 5), (13, 2)])
+def test_frame_batches_and_initial_states(n, batch, dtype):
+    """Per-instance parameters (in_axes) and initial states, and the cotangent
+    of the initial state, against the oracle instance by instance."""
+    body = _circuit(n, n, 40)
+    rng = np.random.default_rng(5 + n)
+    base = rng.uniform(0, 2 * np.pi, (batch, 123))
+    init = rng.normal(size=(batch, 2**n)) + 1j * rng.normal(size=(batch, 2**n))
+    init /= np.linalg.norm(init, axis=1, keepdims=True)
+    obs = [jq.PauliZ(w) for w in range(n)]
+    script = jq.Script(lambda p: body(p) and None, n_qubits=n)
+    params = torch.tensor(base, requires_grad=True)
+    start = torch.tensor(init, requires_grad=True)
+    ev = script.execute("expval", obs, args=(params,), in_axes=(0,), initial_state=start, dtype=dtype)
+    for b in range(batch):
+        recs = to_records(script.record(torch.tensor(base[b])))
+        want = O.expval_state(O.simulate_pure(recs, n, init[b]), n, obs_records(obs))
+        np.testing.assert_allclose(ev[b].detach().cpu().numpy(), want, atol=TOL[dtype], rtol=0)
+    ev.sum().backward()
+    # one parameter and one amplitude of the last instance by central differences
+    h, b = 1e-5, batch - 1
+
+    def total(p, s):
+        return O.expval_state(O.simulate_pure(to_records(script.record(torch.tensor(p))), n, s), n,
+                              obs_records(obs)).sum()
+
+    for k in (0, 7):
+        lo, hi = base[b].copy(), base[b].copy()
+        lo[k] -= h
+        hi[k] += h
+        fd = (total(hi, init[b]) - total(lo, init[b])) / (2 * h)
+        # the difference quotient is good to h^2 n and rounding / h
+        np.testing.assert_allclose(params.grad[b, k].item(), fd, atol=TOL[dtype] * n + 1e-8)
+    lo, hi = init[b].copy(), init[b].copy()
+    lo[3] -= h
+    hi[3] += h
+    fd = (total(base[b], hi) - total(base[b], lo)) / (2 * h)
+    np.testing.assert_allclose(start.grad[b, 3].real.item(), fd, atol=TOL[dtype] * n + 1e-8)
+
+
+def test_frame_plans_run_fewer_passes():
+    """CX rings cost no pass: the 16-qubit ring of 6 layers (96 gates in tiles of
+    11 bits) takes fewer passes than layers x ceil(16 / 8)."""
+    n, layers = 16, 6
+
+    def circuit(p):
+        for l in range(layers):
+            for w in range(n):
+                jq.Rot(p[l, w, 0], p[l, w, 1], p[l, w, 2], wires=w)
+            for w in range(n):
+                jq.CX(wires=[w, (w + 1) % n])
+
+    script = jq.Script(circuit, n_qubits=n)
+    plan = _plan(script, (torch.zeros(layers, n, 3),), [jq.PauliZ(0)], n, torch.complex64)
+    assert plan.info["n_passes_fwd"] < 2 * layers
+    assert plan.info["n_tile_ops_fwd"] == n * layers
