@@ -153,7 +153,13 @@ typedef struct jq_tune {
                             jit 0, 9 qubits or more) moves no amplitude for
                             any permutation: its state buffers hold the
                             amplitudes at linearly mapped indices, up to
-                            signs, for jq_adjoint of the same plan.            */
+                            signs, for jq_adjoint of the same plan.  A density
+                            plan of one-qubit gates, one-qubit channels and
+                            X / CX / SWAP-like permutations with Pauli words
+                            (default tuning, 5 qubits or more) runs
+                            expectation values from |0..0> (init NULL) on
+                            Pauli coefficients; the state buffer then holds
+                            those.                                             */
 } jq_tune;
 
 /* Plan summary. */

@@ -9,13 +9,20 @@ namespace {
 
 int par64(uint64_t v) { return __builtin_popcountll(v) & 1; }
 
+// A gate on n index bits: their masks, functionals and inversions.
 struct Gate {
-  uint32_t m, r;
-  int s;
-  FrameGate fg;
+  int n = 0;
+  uint32_t m[2] = {}, r[2] = {};
+  int s[2] = {};
+  FrameGate fg{};
 };
 
-bool commute(const Gate& a, const Gate& b) { return !par64(a.r & b.m) && !par64(b.r & a.m); }
+bool commute(const Gate& a, const Gate& b) {
+  for (int i = 0; i < a.n; ++i)
+    for (int j = 0; j < b.n; ++j)
+      if (par64(a.r[i] & b.m[j]) || par64(b.r[j] & a.m[i])) return false;
+  return true;
+}
 
 // Span of GF(2) vectors by highest set bit.
 struct Span {
@@ -38,22 +45,25 @@ struct Span {
   }
 };
 
-uint32_t swizzle(uint32_t l, int nbank) {
+// Shared position of tile index l: 16-byte chunks (2^cb values) keep their
+// order inside, the higher bits fold onto the three bank bits of a chunk.
+uint32_t swizzle(uint32_t l, int cb) {
   uint32_t r = l;
-  for (int pos = nbank; pos < 16; ++pos)
-    if (l >> pos & 1u) r ^= 1u << (pos % nbank);
+  for (int pos = cb + 3; pos < 16; ++pos)
+    if (l >> pos & 1u) r ^= 1u << (cb + (pos - cb) % 3);
   return r;
 }
 
 }  // namespace
 
-bool frame_schedule(const std::vector<FrameOp>& ops, int nb, int t_max, int c, int elem, std::vector<uint64_t>* zt,
-                    std::vector<double>* zsign, FramePlan* out) {
+bool frame_schedule(const std::vector<FrameOp>& ops, int nb, int t_max, int c, int elem, int max_st,
+                    std::vector<uint64_t>* zt, std::vector<double>* zsign, FramePlan* out) {
   if (nb < kFrameRB || nb > 31 || t_max < kFrameRB || t_max > kFrameMaxT) return false;
   t_max = std::min(t_max, nb);
   c = std::min(c, t_max);
+  if (c < 2) return false;  // chunks of 16 bytes are contiguous
   // `nbank` lane bits fill a shared-memory wavefront of amplitudes
-  const int esh = elem == 8 ? 3 : 4, nbank = elem == 8 ? 4 : 3;
+  const int esh = elem == 4 ? 2 : elem == 8 ? 3 : 4, nbank = 7 - esh, cb = 4 - esh;
   // ---- gates in the frame ----------------------------------------------------
   std::vector<uint32_t> m(nb), r(nb);
   std::vector<int> s(nb, 0);
@@ -61,7 +71,15 @@ bool frame_schedule(const std::vector<FrameOp>& ops, int nb, int t_max, int c, i
   std::vector<Gate> gates;
   for (const FrameOp& op : ops) {
     if (op.block >= 0) {
-      gates.push_back({m[op.bit[0]], r[op.bit[0]], s[op.bit[0]], op.gate});
+      Gate g;
+      g.n = op.k;
+      for (int i = 0; i < op.k; ++i) {
+        g.m[i] = m[op.bit[i]];
+        g.r[i] = r[op.bit[i]];
+        g.s[i] = s[op.bit[i]];
+      }
+      g.fg = op.gate;
+      gates.push_back(g);
       continue;
     }
     // inverse of the linear part, by elimination on [A | I] (rows = outputs)
@@ -96,6 +114,7 @@ bool frame_schedule(const std::vector<FrameOp>& ops, int nb, int t_max, int c, i
     }
     for (int o = 0; o < k; ++o) { r[op.bit[o]] = rn[o]; m[op.bit[o]] = mn[o]; s[op.bit[o]] = sn[o]; }
   }
+  out->mask = m;
   // Z words over the logical bits -> words over the physical bits
   for (size_t z = 0; z < zt->size(); ++z) {
     uint64_t w = 0;
@@ -115,8 +134,7 @@ bool frame_schedule(const std::vector<FrameOp>& ops, int nb, int t_max, int c, i
   std::vector<int> rem(ngate);
   for (int i = 0; i < ngate; ++i) rem[i] = i;
   size_t head = 0;  // rem[head..] are left
-  const bool whole = t_max == nb;
-  const int max_st = whole ? kFrameMaxStages : kFrameBallot;
+  const int cap = kFrameRB / (gates.empty() ? 1 : gates[0].n);  // gates of a stage
   const size_t window = static_cast<size_t>(4 * nb);
   while (head < rem.size()) {
     Span V;
@@ -129,8 +147,11 @@ bool frame_schedule(const std::vector<FrameOp>& ops, int nb, int t_max, int c, i
       bool ok = true;
       for (int d : deferred)
         if (!commute(gates[g], gates[d])) { ok = false; break; }
-      const bool in = V.reduce(gates[g].m) == 0;
-      if (ok && !in && V.dim >= t_max) ok = false;
+      Span U = V;
+      if (ok) {
+        for (int i = 0; i < gates[g].n; ++i) U.add(gates[g].m[i]);
+        ok = U.dim <= t_max;
+      }
       if (ok) {
         // earliest stage after the last one that holds a gate g must follow
         size_t k = stg.size();
@@ -141,12 +162,12 @@ bool frame_schedule(const std::vector<FrameOp>& ops, int nb, int t_max, int c, i
           if (!dual) break;
           --k;
         }
-        while (k < stg.size() && stg[k].size() >= kFrameRB) ++k;
+        while (k < stg.size() && static_cast<int>(stg[k].size()) >= cap) ++k;
         if (k == stg.size() && static_cast<int>(stg.size()) >= max_st) ok = false;
         if (ok) {
           if (k == stg.size()) stg.emplace_back();
           stg[k].push_back(g);
-          V.add(gates[g].m);
+          V = U;
           members.push_back(g);
         }
       }
@@ -197,13 +218,13 @@ bool frame_schedule(const std::vector<FrameOp>& ops, int nb, int t_max, int c, i
         if (l >> i & 1u) x ^= basis[i];
       return x;
     };
-    auto bytes = [&](uint32_t l) { return swizzle(l, nbank) << esh; };
+    auto bytes = [&](uint32_t l) { return swizzle(l, cb) << esh; };
     // copy vectors: the low unit vectors, then those whose shared offsets add
-    // bank bits to the 16 (8) lanes of a wavefront
+    // bank bits to the 8 lanes of a wavefront of 16-byte chunks
     {
       std::vector<uint32_t> left(basis.begin() + c, basis.end()), order(basis.begin(), basis.begin() + c);
       Span B;
-      const uint32_t wm = 127u;
+      const uint32_t wm = 112u;
       for (uint32_t x : order) B.add(bytes(local(x)) & wm);
       while (!left.empty()) {
         size_t k = 0;
@@ -215,13 +236,15 @@ bool frame_schedule(const std::vector<FrameOp>& ops, int nb, int t_max, int c, i
       }
       for (int i = 0; i < t; ++i) { pd.g[i] = order[i]; pd.cs[i] = bytes(local(order[i])); }
     }
-    // a stage whose functionals vanish on global bits 0 and 1 can keep them as
+    // a stage whose functionals vanish on the lowest index bits can keep them as
     // lane bits: a warp's store then fills whole sectors.  Prefer such a stage
     // last (and, for the adjoint, first) where it commutes past the others.
-    const uint32_t lowm = elem == 8 ? 3u : 1u;
+    const int ns = 5 - esh;  // index bits of a 32-byte sector
+    const uint32_t lowm = (1u << ns) - 1u;
     auto sector = [&](const std::vector<int>& st) {
       for (int g : st)
-        if (gates[g].r & lowm) return false;
+        for (int i = 0; i < gates[g].n; ++i)
+          if (gates[g].r[i] & lowm) return false;
       return true;
     };
     auto passes_by = [&](size_t a, size_t b) {
@@ -251,24 +274,26 @@ bool frame_schedule(const std::vector<FrameOp>& ops, int nb, int t_max, int c, i
     for (size_t k = 0; k < stg.size(); ++k) {
       FrameStage fs;
       std::memset(&fs, 0, sizeof(fs));
-      const int ng = static_cast<int>(stg[k].size());
-      fs.ng = ng;
+      fs.ng = static_cast<int32_t>(stg[k].size());
       uint32_t rho[kFrameRB] = {}, mu[kFrameRB] = {};
       for (int q = 0; q < kFrameRB; ++q) fs.gate[q] = fs.off[q] = -1;
-      for (int q = 0; q < ng; ++q) {
-        const Gate& g = gates[stg[k][q]];
-        mu[q] = local(g.m);
-        if (global(mu[q]) != g.m) return false;
-        for (int i = 0; i < t; ++i) rho[q] |= static_cast<uint32_t>(par64(g.r & basis[i])) << i;
-        fs.r[q] = g.r;
-        if (g.s) fs.sbits |= 1u << q;
+      int ng = 0;  // register bits with a role
+      for (int gi : stg[k]) {
+        const Gate& g = gates[gi];
         FrameGate fg = g.fg;
-        fg.m = g.m;
-        fg.r = g.r;
+        fg.m = g.m[0];
+        fg.r = g.r[0];
         if (fg.grad >= 0) fg.grad = out->n_grad++;
-        fs.gate[q] = fg.grad;
-        fs.off[q] = fg.mat_off;
-        if (fg.diag) fs.diag |= 1 << q;
+        for (int i = 0; i < g.n; ++i, ++ng) {
+          mu[ng] = local(g.m[i]);
+          if (global(mu[ng]) != g.m[i]) return false;
+          for (int q = 0; q < t; ++q) rho[ng] |= static_cast<uint32_t>(par64(g.r[i] & basis[q])) << q;
+          fs.r[ng] = g.r[i];
+          if (g.s[i]) fs.sbits |= 1u << ng;
+          fs.gate[ng] = fg.grad;
+          fs.off[ng] = fg.mat_off;
+          fs.diag |= fg.diag << (2 * ng);
+        }
         out->gates.push_back(fg);
       }
       // kernel of the functionals: projections of the unit vectors
@@ -288,10 +313,10 @@ bool frame_schedule(const std::vector<FrameOp>& ops, int nb, int t_max, int c, i
       const uint32_t bm = (1u << nbank) - 1u;
       std::vector<uint32_t> lanes, rest;
       {
-        uint32_t ev[4] = {}, el[4] = {};  // echelon of bank parts and the vectors behind them
+        uint32_t ev[8] = {}, el[8] = {};  // echelon of bank parts and the vectors behind them
         int ne = 0;
         for (uint32_t x : kb) {
-          uint32_t bx = swizzle(x, nbank) & bm, y = x;
+          uint32_t bx = swizzle(x, cb) & bm, y = x;
           for (int q = 0; q < ne; ++q)
             if (bx & (ev[q] & (~ev[q] + 1u))) { bx ^= ev[q]; y ^= el[q]; }
           if (bx && ne < nbank) {
@@ -319,7 +344,8 @@ bool frame_schedule(const std::vector<FrameOp>& ops, int nb, int t_max, int c, i
       if (static_cast<int>(lanes.size()) != t - kFrameRB) return false;
       for (int q = 0; q < kFrameRB; ++q) { fs.e[q] = bytes(reg[q]); fs.ge[q] = global(reg[q]); }
       for (int i = 0; i < t - kFrameRB; ++i) { fs.tv[i] = bytes(lanes[i]); fs.gtv[i] = global(lanes[i]); }
-      const bool dir = t - kFrameRB >= 2 && fs.gtv[0] == 1u && (elem != 8 || fs.gtv[1] == 2u);
+      bool dir = t - kFrameRB >= ns;
+      for (int i = 0; i < ns && dir; ++i) dir = fs.gtv[i] == 1u << i;
       if (k + 1 == stg.size()) pd.direct = dir;
       if (k == 0) pd.adirect = dir;
       out->stages.push_back(fs);

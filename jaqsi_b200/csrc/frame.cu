@@ -7,33 +7,12 @@
 #include <cstring>
 #include <string>
 
-#include "frame.h"
+#include "frame_dev.cuh"
 #include "jq_internal.h"
 #include "kernels.cuh"
 
 namespace jq {
-void set_error(const std::string& msg);
-
 namespace {
-
-#define JQ_CUDA(expr)                                                                       \
-  do {                                                                                      \
-    cudaError_t _e = (expr);                                                                \
-    if (_e != cudaSuccess) {                                                                \
-      set_error(std::string("CUDA error: ") + cudaGetErrorString(_e) + " at " #expr);       \
-      return JQ_ECUDA;                                                                      \
-    }                                                                                       \
-  } while (0)
-
-// Kernel argument of one pass.
-struct PassArg {
-  uint32_t g[kFrameMaxT];
-  uint32_t cs[kFrameMaxT];
-  uint32_t opos[32];
-  int32_t nb, nouter, c;
-  int32_t st0, nst;
-  int32_t direct;
-};
 
 // Gate parameters.
 //
@@ -83,15 +62,6 @@ template <typename C> struct TabOf;
 template <> struct TabOf<float2> { using T = Tab32; };
 template <> struct TabOf<double2> { using T = Tab64; };
 template <typename C> using Tab = typename TabOf<C>::T;
-
-__device__ __forceinline__ void cp_async(uint32_t sa, const float2* g) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(g) : "memory");
-}
-__device__ __forceinline__ void cp_async(uint32_t sa, const double2* g) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(g) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 __device__ __forceinline__ void rot_pair(double2& x, double2& y, double t) {
   const double2 a = x;
@@ -179,46 +149,9 @@ __device__ __forceinline__ void mul_all(float2 (&v)[16], float f) {
 }
 __device__ __forceinline__ void mul_all(double2 (&)[16], double) {}
 
-// Shared-memory accesses by byte offset; two tiles lie at offsets 0 and 2^T
-// amplitudes, so that tile, thread and slot parts of an offset combine by XOR.
-extern __shared__ __align__(16) unsigned char smem[];
-template <typename C> __device__ __forceinline__ C lds(uint32_t a) { return *reinterpret_cast<const C*>(smem + a); }
-template <typename C> __device__ __forceinline__ void sts(uint32_t a, C v) { *reinterpret_cast<C*>(smem + a) = v; }
-
-// Offset of register slot j = XOR of the register vectors of its bits.
-__device__ __forceinline__ void slot_offsets(const uint32_t (&e)[4], uint32_t base, uint32_t (&a)[16]) {
-  a[0] = base;
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-#pragma unroll
-    for (int j = 0; j < (1 << q); ++j) a[j | (1 << q)] = a[j] ^ e[q];
-}
-__device__ __forceinline__ uint32_t slot_xor(const uint32_t* e, uint32_t n) {
-  return ((n & 1u) ? e[0] : 0u) ^ ((n & 2u) ? e[1] : 0u) ^ ((n & 4u) ? e[2] : 0u) ^ ((n & 8u) ? e[3] : 0u);
-}
-
 // Shared-memory plan of a pass, in bytes.
 template <typename C>
 __host__ __device__ constexpr size_t tab_bytes(int nst) { return static_cast<size_t>(nst) * sizeof(Tab<C>); }
-__host__ __device__ constexpr size_t soff_bytes(int nst) { return static_cast<size_t>(nst) * 16 * sizeof(uint32_t); }
-__host__ __device__ constexpr size_t tb_bytes(int nst, int threads) {
-  return (static_cast<size_t>(nst) * threads * sizeof(uint16_t) + 15) & ~static_cast<size_t>(15);
-}
-
-// Tile-independent offsets of a pass: thread bases (in 8 bytes) and slots.
-template <int LT>
-__device__ __forceinline__ void pass_setup(const FrameStage* __restrict__ st, int nst, uint16_t* tbs, uint32_t* soff) {
-  const uint32_t tid = threadIdx.x;
-  for (int k = 0; k < nst; ++k) {
-    uint32_t b = 0;
-#pragma unroll
-    for (int i = 0; i < LT; ++i)
-      if (tid >> i & 1u) b ^= st[k].tv[i];
-    tbs[k * (1 << LT) + tid] = static_cast<uint16_t>(b >> 3);
-  }
-  for (int i = tid; i < nst * 16; i += 1 << LT) soff[i] = slot_xor(st[i >> 4].e, i & 15);
-}
-
 // Stage tables of one instance.
 template <int LT>
 __device__ __forceinline__ void pass_tables(const FrameStage* __restrict__ st, int nst, const float2* __restrict__ bm, Tab32* tab) {
@@ -230,7 +163,7 @@ __device__ __forceinline__ void pass_tables(const FrameStage* __restrict__ st, i
       float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
       float2 h = make_float2(0.f, 0.f);
       if (j < s.ng) {
-        const bool diag = s.diag >> j & 1;
+        const bool diag = s.diag >> (2 * j) & 1;
         const Gate32* m = gate_at(bm, s.off[j], diag);
         if (!diag) g = make_float4(m->t, m->tau0, m->sig0, 0.f);
         h = make_float2(m->tau1, m->sig1);
@@ -239,14 +172,14 @@ __device__ __forceinline__ void pass_tables(const FrameStage* __restrict__ st, i
       tb.h[j] = h;
     } else if (j == 4) {
       uint32_t piv = 0;
-      for (int q = 0; q < s.ng; ++q) piv |= (gate_flags(bm, s.off[q], s.diag >> q & 1) & 1u) << q;
+      for (int q = 0; q < s.ng; ++q) piv |= (gate_flags(bm, s.off[q], s.diag >> (2 * q) & 1) & 1u) << q;
       tb.piv = piv;
     } else if (j == 5) {
       double f = 1.0;
       const int k = i >> 3, k1 = min(nst, (k | 3) + 1);
       for (int x = k; x < k1; ++x)
         for (int q = 0; q < st[x].ng; ++q)
-          if (!(st[x].diag >> q & 1)) {
+          if (!(st[x].diag >> (2 * q) & 1)) {
             const double t = gate_at(bm, st[x].off[q], false)->t;  // the rounded one: exactly its norm
             f *= 1.0 + t * t;
           }
@@ -263,27 +196,20 @@ __device__ __forceinline__ void pass_tables(const FrameStage* __restrict__ st, i
     double2 pre = make_double2(1, 0), post = make_double2(1, 0);
     for (int q = 0; q < s.ng; ++q) {
       const double2* m = bm + s.off[q];
-      const bool hi = j >> q & 1, diag = s.diag >> q & 1;
+      const bool hi = j >> q & 1, diag = s.diag >> (2 * q) & 1;
       post = cmul(post, m[hi ? 1 : 0]);
       if (!diag && hi) pre = cmul(pre, m[2]);
     }
     Tab64& tb = tab[i >> 4];
     tb.pre[j] = pre;
     tb.post[j] = post;
-    if (j < 4) tb.t[j] = (j < s.ng && !(s.diag >> j & 1)) ? bm[s.off[j] + 3].x : 0.0;
+    if (j < 4) tb.t[j] = (j < s.ng && !(s.diag >> (2 * j) & 1)) ? bm[s.off[j] + 3].x : 0.0;
     if (j == 4) {
       uint32_t piv = 0;
-      for (int q = 0; q < s.ng; ++q) piv |= gate_flags(bm, s.off[q], s.diag >> q & 1) << q;
+      for (int q = 0; q < s.ng; ++q) piv |= gate_flags(bm, s.off[q], s.diag >> (2 * q) & 1) << q;
       tb.piv = piv;
     }
   }
-}
-
-// Representative of tile ti: its index bits at the free positions.
-__device__ __forceinline__ uint32_t tile_rep(uint64_t ti, uint32_t opos_lane, int nouter) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t v = (lane < nouter && (ti >> lane & 1ULL)) ? opos_lane : 0u;
-  return __reduce_or_sync(0xffffffffu, v);
 }
 
 // One forward pass.  A tile (a coset of V) streams into shared memory while
@@ -292,9 +218,10 @@ __device__ __forceinline__ uint32_t tile_rep(uint64_t ti, uint32_t opos_lane, in
 //
 // Bound by instruction issue and its latencies (58% of issue slots, 120
 // instructions an amplitude and pass of 14 gates, 65 of them FP32; shared memory
-// 51%, HBM 40% busy).  24 qubits, 20 layers, complex64: 34 to 40 passes of 105 us
-// for 133 stages against 66 passes of 60 us for 157, 4.20 -> 3.55 ms a call.  Five
-// CTAs an SM; six (79 registers) 4.19 ms.  Pairs of amplitudes in packed FMAs
+// 51%, HBM 40% busy).  24 qubits, 20 layers, complex64: 40 passes of 80 us for 133
+// stages against 66 passes of 60 us for 157, 4.20 -> 3.28 ms a call (3.55 with
+// tiles copied 8 bytes at a time instead of 16).  Five CTAs an SM; six (79
+// registers) were 18% slower.  Pairs of amplitudes in packed FMAs
 // throughout: 1.5 times slower, register moves for every packed operand.
 template <typename C, int T, int MINB>
 __global__ void __launch_bounds__(1 << (T - 4), MINB)
@@ -314,31 +241,18 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
   const uint32_t opos_lane = P.opos[lane];
   const uint32_t r_lane = (lane >> 2) < static_cast<uint32_t>(nst) ? st[lane >> 2].r[lane & 3] : 0u;
   const uint32_t s_lane = (lane >> 2) < static_cast<uint32_t>(nst) ? (st[lane >> 2].sbits >> (lane & 3) & 1u) : 0u;
-  // global offsets: this thread's part, and the 16 rows of the copy
-  uint32_t gtid = 0, gout = 0;
+  uint32_t gout = 0;  // this thread's part of the last stage's indices
 #pragma unroll
   for (int i = 0; i < LT; ++i)
-    if (tid >> i & 1u) {
-      gtid ^= P.g[i];
-      gout ^= st[nst - 1].gtv[i];
-    }
-  uint32_t stid = 0;
-#pragma unroll
-  for (int i = 0; i < LT; ++i)
-    if (tid >> i & 1u) stid ^= P.cs[i];
-  const uint32_t sq[4] = {P.cs[LT], P.cs[LT + 1], P.cs[LT + 2], P.cs[LT + 3]};
-  const uint32_t gq[4] = {P.g[LT], P.g[LT + 1], P.g[LT + 2], P.g[LT + 3]};
+    if (tid >> i & 1u) gout ^= st[nst - 1].gtv[i];
+  const TileCopy<C, LT> copy(P);
   const uint64_t tiles_per = 1ULL << P.nouter;
   const int64_t ntiles = static_cast<int64_t>(tiles_per) * batch;
   const uint64_t rmask = rev ? tiles_per - 1 : 0;
   auto load = [&](uint32_t dst, int64_t tl) {
     const uint32_t rep = tile_rep((static_cast<uint64_t>(tl) & (tiles_per - 1)) ^ rmask, opos_lane, P.nouter);
     const C* src = state + ((tl >> P.nouter) << P.nb);
-    uint32_t a[16], b[16];
-    slot_offsets(gq, rep ^ gtid, a);
-    slot_offsets(sq, dst ^ stid, b);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) cp_async(sbase + b[i], src + a[i]);
+    copy.each(P, rep, dst, [&](uint32_t a, uint32_t b) { cp_async16(sbase + b, src + a); });
   };
   __syncthreads();
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -365,7 +279,7 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
       const uint32_t nib = k < kFrameBallot ? (flips >> (4 * k)) & 15u : st[k].sbits;
       const uint32_t* so = soff + 16 * k;
       const uint32_t e[4] = {so[1], so[2], so[4], so[8]};
-      const uint32_t base = s ^ (static_cast<uint32_t>(tbs[k * NT + tid]) << 3);
+      const uint32_t base = s ^ (static_cast<uint32_t>(tbs[k * NT + tid]) << 2);
       uint32_t a[16];
       C v[16];
       slot_offsets(e, base ^ so[nib ^ tb.piv], a);
@@ -388,34 +302,12 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
       }
     }
     if (!P.direct) {
-      uint32_t a[16], b[16];
-      slot_offsets(gq, rep ^ gtid, a);
-      slot_offsets(sq, s ^ stid, b);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) __stcs(g + a[i], lds<C>(b[i]));
+      copy.each(P, rep, s, [&](uint32_t a, uint32_t b) { __stcs(reinterpret_cast<float4*>(g + a), lds<float4>(b)); });
     }
     __syncthreads();
     s ^= TB;
   }
 }
-
-// Warp reduce-scatter of 16 per-lane sums by recursive halving (16 shuffles);
-// even lane 2 v ends with the sum of value v.
-template <typename F>
-__device__ __forceinline__ F warp_rs16(F (&v)[16], unsigned lane) {
-#pragma unroll
-  for (int o = 16, n = 16; o > 1; o >>= 1, n >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int i = 0; i < n / 2; ++i) {
-      const F send = up ? v[i] : v[i + n / 2];
-      const F keep = up ? v[i + n / 2] : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-  }
-  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
-}
-
 
 // One adjoint pass: the pass's stages in reverse on psi and lambda, and the three
 // components Im tr(sigma_k lam psi^dagger) of each gate's cotangent, all four
@@ -423,7 +315,7 @@ __device__ __forceinline__ F warp_rs16(F (&v)[16], unsigned lane) {
 // other gates of its stage, and the generators of a rotation see only these
 // three of its eight numbers.  Partial sums in the run precision per tile and
 // warp, float64 across tiles.  20 qubits, 50 layers, complex64 (forward +
-// adjoint): 4.77 -> 3.65 ms a call; 16 qubits, 9 layers, complex128, three sets:
+// adjoint): 4.77 -> 3.42 ms a call; 16 qubits, 9 layers, complex128, three sets:
 // 0.93 -> 0.75 ms.
 template <typename C, int T, int MINB>
 __global__ void __launch_bounds__(1 << (T - 4), MINB)
@@ -445,19 +337,11 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
   const uint32_t opos_lane = P.opos[lane];
   const uint32_t r_lane = (lane >> 2) < static_cast<uint32_t>(nst) ? st[lane >> 2].r[lane & 3] : 0u;
   const uint32_t s_lane = (lane >> 2) < static_cast<uint32_t>(nst) ? (st[lane >> 2].sbits >> (lane & 3) & 1u) : 0u;
-  uint32_t gtid = 0, gout = 0;
+  uint32_t gout = 0;
 #pragma unroll
   for (int i = 0; i < LT; ++i)
-    if (tid >> i & 1u) {
-      gtid ^= P.g[i];
-      gout ^= st[0].gtv[i];
-    }
-  uint32_t stid = 0;
-#pragma unroll
-  for (int i = 0; i < LT; ++i)
-    if (tid >> i & 1u) stid ^= P.cs[i];
-  const uint32_t sq[4] = {P.cs[LT], P.cs[LT + 1], P.cs[LT + 2], P.cs[LT + 3]};
-  const uint32_t gq[4] = {P.g[LT], P.g[LT + 1], P.g[LT + 2], P.g[LT + 3]};
+    if (tid >> i & 1u) gout ^= st[0].gtv[i];
+  const TileCopy<C, LT> copy(P);
   const uint64_t tiles_per = 1ULL << P.nouter;
   const int64_t ntiles = static_cast<int64_t>(tiles_per) * batch;
   int64_t last = -1;
@@ -477,17 +361,11 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
     const uint32_t flips = __ballot_sync(0xffffffffu, ((__popc(rep & r_lane) & 1u) ^ s_lane) != 0u);
     const int64_t ibase = inst << P.nb;
     __syncthreads();
-    {
-      uint32_t a[16], b[16];
-      slot_offsets(gq, rep ^ gtid, a);
-      slot_offsets(sq, stid, b);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        cp_async(sbase + b[i], psi_in + ibase + a[i]);
-        cp_async(sbase + (b[i] ^ TB), lam + ibase + a[i]);
-      }
-      cp_commit();
-    }
+    copy.each(P, rep, 0, [&](uint32_t a, uint32_t b) {
+      cp_async16(sbase + b, psi_in + ibase + a);
+      cp_async16(sbase + (b ^ TB), lam + ibase + a);
+    });
+    cp_commit();
     if (inst != last) {
       if (last >= 0) {
         flush(last);
@@ -502,7 +380,7 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
     for (int k = nst - 1; k >= 0; --k) {
       const Tab<C>& tb = tab[k];
       const uint32_t nib = k < kFrameBallot ? (flips >> (4 * k)) & 15u : st[k].sbits;
-      const uint32_t base = static_cast<uint32_t>(tbs[k * NT + tid]) << 3;
+      const uint32_t base = static_cast<uint32_t>(tbs[k * NT + tid]) << 2;
       const uint32_t* so = soff + 16 * k;
       const uint32_t e[4] = {so[1], so[2], so[4], so[8]};
       C p[16], l[16];
@@ -572,14 +450,10 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
       if (!(P.direct && k == 0)) __syncthreads();
     }
     if (!P.direct) {
-      uint32_t a[16], b[16];
-      slot_offsets(gq, rep ^ gtid, a);
-      slot_offsets(sq, stid, b);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        __stcs(psi + ibase + a[i], lds<C>(b[i]));
-        __stcs(lam + ibase + a[i], lds<C>(b[i] ^ TB));
-      }
+      copy.each(P, rep, 0, [&](uint32_t a, uint32_t b) {
+        __stcs(reinterpret_cast<float4*>(psi + ibase + a), lds<float4>(b));
+        __stcs(reinterpret_cast<float4*>(lam + ibase + a), lds<float4>(b ^ TB));
+      });
     }
   }
   __syncthreads();
@@ -778,11 +652,6 @@ __global__ void k_frame_chain(const FrameGate* __restrict__ gates, int ngates, c
 }
 
 // ---- launches ------------------------------------------------------------------
-bool pdl_on(cudaStream_t st) {
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
-}
-
 template <typename C, int T> constexpr int fwd_minb() {
   // 128 threads (11 bits): complex64 5 CTAs an SM (100 registers), complex128 3 (168)
   return sizeof(C) == 8 ? (T >= 12 ? 2 : T == 11 ? 5 : 8) : (T >= 12 ? 1 : T == 11 ? 3 : 6);
@@ -816,21 +685,6 @@ template <typename C> const void* adj_kernel(const FramePass& p) {
     case 11: return reinterpret_cast<const void*>(&k_frame_adj<C, 11, adj_minb<C, 11>()>);
     default: return reinterpret_cast<const void*>(&k_frame_adj<C, 12, adj_minb<C, 12>()>);
   }
-}
-
-PassArg pass_arg(const FramePass& p, int nb, bool adjoint) {
-  PassArg a;
-  std::memset(&a, 0, sizeof(a));
-  std::memcpy(a.g, p.g, sizeof(a.g));
-  std::memcpy(a.cs, p.cs, sizeof(a.cs));
-  std::memcpy(a.opos, p.opos, sizeof(a.opos));
-  a.nb = nb;
-  a.nouter = p.nouter;
-  a.c = p.c;
-  a.st0 = p.st0;
-  a.nst = p.nst;
-  a.direct = adjoint ? p.adirect : p.direct;
-  return a;
 }
 
 template <typename C> int upload_shapes(const FramePlan& fp, FrameDev* d) {
@@ -895,9 +749,7 @@ int adjoint_t(const jq_plan* plan, const FrameDev& d, const C* psi_in, C* psi, C
 
 }  // namespace
 
-int frame_upload(const jq_plan* plan, FrameDev* d) {
-  const FramePlan& fp = plan->frame;
-  if (!fp.on) return JQ_OK;
+int frame_tables(const FramePlan& fp, FrameDev* d) {
   const size_t ns = std::max<size_t>(1, fp.stages.size()), ng = std::max<size_t>(1, fp.gates.size());
   JQ_CUDA(cudaMalloc(reinterpret_cast<void**>(&d->stages), ns * sizeof(FrameStage)));
   JQ_CUDA(cudaMalloc(reinterpret_cast<void**>(&d->gates), ng * sizeof(FrameGate)));
@@ -905,6 +757,14 @@ int frame_upload(const jq_plan* plan, FrameDev* d) {
     JQ_CUDA(cudaMemcpy(d->stages, fp.stages.data(), fp.stages.size() * sizeof(FrameStage), cudaMemcpyHostToDevice));
   if (!fp.gates.empty())
     JQ_CUDA(cudaMemcpy(d->gates, fp.gates.data(), fp.gates.size() * sizeof(FrameGate), cudaMemcpyHostToDevice));
+  return JQ_OK;
+}
+
+int frame_upload(const jq_plan* plan, FrameDev* d) {
+  const FramePlan& fp = plan->frame;
+  if (!fp.on) return JQ_OK;
+  const int rc = frame_tables(fp, d);
+  if (rc) return rc;
   return plan->dtype == JQ_C64 ? upload_shapes<float2>(fp, d) : upload_shapes<double2>(fp, d);
 }
 

@@ -33,6 +33,7 @@ namespace jq {
 struct DevBlock;
 struct DevPrim;
 struct DevOp;
+struct DeviceTables;
 
 constexpr int kFrameMaxT = 12;      // largest tile (2^12 amplitudes)
 constexpr int kFrameRB = 4;         // gates of a stage, register slots 2^4
@@ -42,7 +43,7 @@ constexpr int kFrameMaxStages = 24; // stages of a pass that holds the whole sta
 struct FrameGate {
   int32_t block;     // fused block of the plan
   int32_t mat_off;   // its parameters in the block-matrix row (run-dtype complex elements)
-  int32_t diag;      // 1: diagonal block (two elements), else four
+  int32_t diag;      // 1: diagonal block (statevectors: two elements, else four)
   int32_t grad;      // index among the gates with cotangents, -1: none wanted
   uint32_t m, r;     // mask and role functional
 };
@@ -59,7 +60,7 @@ struct FrameStage {
   int32_t ng;                         // gates
   int32_t gate[kFrameRB];             // cotangent index of the gates, -1 none
   int32_t off[kFrameRB];              // mat_off of the gates, -1 none
-  int32_t diag;                       // bit q: gate q diagonal
+  int32_t diag;                       // bits 2 q: FrameGate::diag of register bit q
 };
 
 struct FramePass {
@@ -79,6 +80,7 @@ struct FramePlan {
   int n_grad = 0;  // gates with cotangents
   std::vector<FrameStage> stages;
   std::vector<FramePass> passes;
+  std::vector<uint32_t> mask;  // final mask of every logical bit
 };
 
 // Uploaded tables and launch shapes of a frame plan on one device.
@@ -90,7 +92,7 @@ struct FrameDev {
 
 // A gate or an affine permutation in program order, as the planner sees it.
 struct FrameOp {
-  int block = -1;                 // >= 0: one-wire gate
+  int block = -1;                 // >= 0: a gate on k = 1 or 2 bits (the same k in one schedule)
   int k = 0;
   int bit[8] = {};                // flat bit of local bit i
   uint32_t col[8] = {};           // permutation: P(x) = xor of col[i] over set bits ^ b
@@ -98,13 +100,15 @@ struct FrameOp {
   FrameGate gate{};
 };
 
-// Schedules ops on nb index bits into passes of at most t_max bits holding the
-// lowest c bits, for amplitudes of `elem` bytes.  zt / zsign: Z words over logical flat bits, rewritten to
-// words over physical bits.  False when a size is out of range.
-bool frame_schedule(const std::vector<FrameOp>& ops, int nb, int t_max, int c, int elem, std::vector<uint64_t>* zt,
-                    std::vector<double>* zsign, FramePlan* out);
+// Schedules ops on nb index bits into passes of at most t_max bits that hold the
+// lowest c bits, and at most max_st stages, for values of `elem` bytes.  zt / zsign:
+// Z words over logical flat bits, rewritten to words over physical bits.  False
+// when a size is out of range.
+bool frame_schedule(const std::vector<FrameOp>& ops, int nb, int t_max, int c, int elem, int max_st,
+                    std::vector<uint64_t>* zt, std::vector<double>* zsign, FramePlan* out);
 
 int frame_upload(const jq_plan* plan, FrameDev* d);
+int frame_tables(const FramePlan& fp, FrameDev* d);  // the tables alone
 void frame_free(FrameDev* d);
 int frame_prep(const jq_plan* plan, const FrameDev& d, const DevBlock* blocks, const DevPrim* prims, const DevOp* ops,
                const double* cpool, int batch, const double* angles, void* bmat, cudaStream_t st);
@@ -117,5 +121,22 @@ int frame_adjoint(const jq_plan* plan, const FrameDev& d, const void* psi_in, vo
 int frame_chain(const jq_plan* plan, const FrameDev& d, const DevBlock* blocks, const DevPrim* prims, const DevOp* ops,
                 const double* cpool, int batch, const double* angles, const void* bmat, const double* gacc,
                 int64_t gstride, double* grad_angles, cudaStream_t st);
+
+// ---- noisy circuits in the Pauli basis (pauli.cu) -----------------------------
+// An observable: coefficient `index` (physical, sign included) times coeff.
+struct PauliObs {
+  uint32_t index;
+  double coeff;
+};
+
+int pauli_upload(const jq_plan* plan, FrameDev* d);
+// state: the coefficients, half a density matrix's bytes.
+int pauli_forward(const jq_plan* plan, const DeviceTables& T, int batch, const double* angles, void* state, void* bmat,
+                  double* out, int sm_count, cudaStream_t st);
+// gacc: 12 doubles a gate with cotangents; slots: n_slots >= 3 states of 256-byte
+// aligned coefficients for pass inputs and checkpoints.
+int pauli_backward(const jq_plan* plan, const DeviceTables& T, int batch, const double* angles, void* bmat, double* gacc,
+                   void* lam, void* slots, int64_t n_slots, const double* ct, double* grad_angles, int sm_count,
+                   cudaStream_t st);
 
 }  // namespace jq

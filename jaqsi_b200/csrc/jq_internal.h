@@ -153,6 +153,8 @@ struct DeviceTables {
   void* obs_desc = nullptr;       // DevObs array
   FrameDev frame;                 // frame plan (plan->frame.on)
   void* frame_obs = nullptr;      // DevObs array over physical bits
+  FrameDev pauli;                 // Pauli-basis plan (plan->pauli.on)
+  void* pauli_obs = nullptr;      // PauliObs array
   void* jit = nullptr;            // JitModule of the forward schedule (or nullptr)
   bool jit_tried = false;
   int jit_rc = 0;                 // nonzero: the required specialisation failed
@@ -189,6 +191,9 @@ struct jq_plan {
   std::vector<double> obs_pool;
   jq::FramePlan frame;               // expectation-value plans of one-wire unitaries and affine permutations
   std::vector<jq::DevObs> frame_obs; // their Z words over physical bits
+  jq::FramePlan pauli;               // density plans of one-qubit gates and channels and linear permutations,
+                                     // run for Pauli expectation values from |0..0>
+  std::vector<jq::PauliObs> pauli_obs;
   jq::Schedule fwd, adj, bwd;  // bwd: one block per pass (the unfused order; diagnostics)
   int64_t bmat_stride = 0;     // run-dtype complex elements per instance
   int64_t grad_stride = 0;     // complex128 elements per instance

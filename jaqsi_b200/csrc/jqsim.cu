@@ -2070,13 +2070,40 @@ int upload(const std::vector<T>& v, T** dst) {
   return JQ_OK;
 }
 
-int device_tables(const jq_plan* cplan, const DeviceTables** out) {
+// The plan's NVRTC specialisation on the current device.
+void build_jit(const jq_plan* plan, DeviceTables* t) {
+  t->jit_tried = true;
+  if (plan->jit && !plan->frame.on && jit_available()) {
+    JitModule* jm = new JitModule();
+    const int rc = jit_build(plan, plan->fwd, jm);
+    if (rc == JQ_OK) {
+      t->jit = jm;
+    } else {
+      jit_free(jm);
+      delete jm;
+      // automatic mode: the register-stage interpreter kernels run instead;
+      // jq_tune.jit = 1: the plan fails on this device (tables kept for jq_plan_free)
+      if (plan->jit_required) {
+        t->jit_rc = rc;
+        t->jit_err = g_last_error;
+      }
+    }
+  } else if (plan->jit_required) {
+    t->jit_rc = JQ_EUNSUPPORTED;
+    t->jit_err = "jq_tune.jit = 1 but NVRTC or the CUDA driver entry points are not available";
+  }
+}
+
+// general: the call runs the general passes (a Pauli-basis plan compiles their
+// specialisation on the first such call only)
+int device_tables(const jq_plan* cplan, const DeviceTables** out, bool general = true) {
   jq_plan* plan = const_cast<jq_plan*>(cplan);
   int dev = 0;
   JQ_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lock(g_upload_mu);
-  for (const DeviceTables& t : plan->dev)
+  for (DeviceTables& t : plan->dev)
     if (t.device == dev) {
+      if (general && !t.jit_tried) build_jit(plan, &t);
       if (t.jit_rc) {
         set_error(t.jit_err);
         return t.jit_rc;
@@ -2105,31 +2132,19 @@ int device_tables(const jq_plan* cplan, const DeviceTables** out) {
   if ((rc = upload(plan->fwd.rops, &t.fwd_rops))) return rc;
   if ((rc = upload(plan->bwd.steps, &t.bwd_steps))) return rc;
   if ((rc = upload(plan->bwd.rops, &t.bwd_rops))) return rc;
-  if (plan->jit && !plan->frame.on && jit_available()) {
-    JitModule* jm = new JitModule();
-    if ((rc = jit_build(plan, plan->fwd, jm)) == JQ_OK) {
-      t.jit = jm;
-    } else {
-      jit_free(jm);
-      delete jm;
-      // automatic mode: the register-stage interpreter kernels run instead;
-      // jq_tune.jit = 1: the plan fails on this device (tables kept for jq_plan_free)
-      if (plan->jit_required) {
-        t.jit_rc = rc;
-        t.jit_err = g_last_error;
-      }
-    }
-  } else if (plan->jit_required) {
-    t.jit_rc = JQ_EUNSUPPORTED;
-    t.jit_err = "jq_tune.jit = 1 but NVRTC or the CUDA driver entry points are not available";
-  }
+  if (general || !plan->pauli.on) build_jit(plan, &t);
   if (plan->frame.on) {
     if ((rc = frame_upload(plan, &t.frame))) return rc;
     DevObs* fo = nullptr;
     if ((rc = upload(plan->frame_obs, &fo))) return rc;
     t.frame_obs = fo;
   }
-  t.jit_tried = true;
+  if (plan->pauli.on) {
+    if ((rc = pauli_upload(plan, &t.pauli))) return rc;
+    PauliObs* po = nullptr;
+    if ((rc = upload(plan->pauli_obs, &po))) return rc;
+    t.pauli_obs = po;
+  }
   plan->dev.push_back(t);
   if (t.jit_rc) {
     set_error(t.jit_err);
@@ -2159,7 +2174,8 @@ WsLayout layout(const jq_plan* plan, int batch, int mode_grad /*0 fwd, 1 adjoint
     L.lam = off;
     off += align256(state);
     L.gacc = off;
-    off += align256(static_cast<size_t>(plan->grad_stride) * 16 * batch);
+    off += align256(std::max(static_cast<size_t>(plan->grad_stride) * 16,
+                             static_cast<size_t>(plan->pauli.n_grad) * 12 * sizeof(double)) * batch);
   }
   if (mode_grad == 1) {
     L.psi = off;
@@ -2177,6 +2193,17 @@ WsLayout layout(const jq_plan* plan, int batch, int mode_grad /*0 fwd, 1 adjoint
     off += align256(state) * static_cast<size_t>(std::max<int64_t>(L.n_ckpt, 1));
     L.seg = off;
     off += align256(state) * static_cast<size_t>(S);
+    if (plan->pauli.on) {
+      // half-size states: every pass input while that takes 256 MB or half as much
+      // again as the general passes at most, two levels of checkpoints at least
+      const size_t half = align256(state / 2);
+      const int64_t Q = static_cast<int64_t>(plan->pauli.passes.size());
+      int64_t two = Q;
+      for (int64_t s = 1; s < Q; ++s) two = std::min(two, (Q + s - 1) / s + s);
+      const size_t all = static_cast<size_t>(Q) * half;
+      const int64_t need = all <= (size_t{256} << 20) || L.work + all <= off + off / 2 ? Q : two;
+      off = std::max(off, L.work + half * static_cast<size_t>(std::max<int64_t>(need, 1)));
+    }
   }
   L.total = off;
   return L;
@@ -2360,13 +2387,20 @@ int measure(const jq_plan* plan, const DeviceTables* T, int batch, int out_type,
   return JQ_OK;
 }
 
+// Whether a call of a Pauli-basis plan runs there: expectation values from
+// |0..0> (an initial state or matrix goes through the general passes).
+bool pauli_call(const jq_plan* plan, int out_type, const void* init) {
+  return plan->pauli.on && out_type == JQ_OUT_EXPVAL && !init;
+}
+
 template <typename R>
 int forward_impl(const jq_plan* plan, int batch, const double* angles, const void* mats, const void* init,
                  int init_batched, int out_type, void* state, void* out, void* ws, size_t ws_bytes,
                  cudaStream_t st) {
   using C = typename CplxT<R>::T;
   const DeviceTables* T = nullptr;
-  int rc = device_tables(plan, &T);
+  const bool pauli = pauli_call(plan, out_type, init);
+  int rc = device_tables(plan, &T, !pauli);
   if (rc) return rc;
   if ((rc = set_smem_attrs<R>())) return rc;
   WsLayout L = layout(plan, batch, 0);
@@ -2376,6 +2410,7 @@ int forward_impl(const jq_plan* plan, int batch, const double* angles, const voi
   }
   char* w = static_cast<char*>(ws);
   C* bmat = reinterpret_cast<C*>(w + L.bmat);
+  if (pauli) return pauli_forward(plan, *T, batch, angles, state, bmat, static_cast<double*>(out), sm_count(), st);
   double2* scratch = reinterpret_cast<double2*>(w + L.scratch);
   if ((rc = prep<R>(plan, T, batch, angles, mats, bmat, scratch, st))) return rc;
   C* S = static_cast<C*>(state);
@@ -2579,13 +2614,25 @@ int backward_impl(const jq_plan* plan, int batch, const double* angles, const vo
                   void* grad_mats, void* grad_init, void* ws, size_t ws_bytes, cudaStream_t st) {
   using C = typename CplxT<R>::T;
   const DeviceTables* T = nullptr;
-  int rc = device_tables(plan, &T);
+  const bool pauli = pauli_call(plan, out_type, init) && !grad_init;
+  int rc = device_tables(plan, &T, !pauli);
   if (rc) return rc;
   if ((rc = set_smem_attrs<R>())) return rc;
   WsLayout L = layout(plan, batch, 2);
   if (ws_bytes < L.total || !ws) {
     set_error("workspace too small: need " + std::to_string(L.total) + " bytes");
     return JQ_ENOMEM;
+  }
+  if (pauli) {
+    char* wp = static_cast<char*>(ws);
+    // the coefficients take half a state; everything behind lambda but the
+    // cotangents holds pass inputs
+    const size_t half = align256(static_cast<size_t>(plan->state_elems) * sizeof(R) * batch);
+    const int64_t n_slots = static_cast<int64_t>((L.total - L.work) / half);
+    if (grad_mats && plan->n_mats > 0)
+      JQ_CUDA(cudaMemsetAsync(grad_mats, 0, 16 * static_cast<size_t>(plan->n_mats) * batch, st));
+    return pauli_backward(plan, *T, batch, angles, wp + L.bmat, reinterpret_cast<double*>(wp + L.gacc), wp + L.lam,
+                          wp + L.work, n_slots, ct, grad_angles, sm_count(), st);
   }
   char* w = static_cast<char*>(ws);
   C* bmat = reinterpret_cast<C*>(w + L.bmat);
@@ -2815,6 +2862,8 @@ int jq_plan_free(jq_plan* plan) {
     cudaFree(t.const_pool);
     frame_free(&t.frame);
     cudaFree(t.frame_obs);
+    frame_free(&t.pauli);
+    cudaFree(t.pauli_obs);
     if (t.jit) {
       jit_free(static_cast<JitModule*>(t.jit));
       delete static_cast<JitModule*>(t.jit);

@@ -154,6 +154,56 @@ bool affine_perm(const HostBlock& hb, int nb, FrameOp* f) {
   return true;
 }
 
+// The same permutation |v> -> |A v> on Pauli words, X^x Z^z -> X^{A x} Z^{A^-T z}
+// (x bit 2 (n-1-w), z bit 2 (n-1-w) + 1); false unless it is linear.
+bool pauli_perm(const HostBlock& hb, int n, FrameOp* f) {
+  const int k = static_cast<int>(hb.wires.size());
+  FrameOp a;
+  if (k > 4 || !affine_perm(hb, n, &a) || a.b != 0) return false;
+  // inverse of A by brute force over its images
+  uint32_t inv[4] = {};  // A^-1 of unit vector o
+  for (uint32_t x = 0; x < (1u << k); ++x) {
+    uint32_t y = 0;
+    for (int i = 0; i < k; ++i)
+      if (x >> i & 1u) y ^= a.col[i];
+    for (int o = 0; o < k; ++o)
+      if (y == 1u << o) inv[o] = x;
+  }
+  f->block = -1;
+  f->k = 2 * k;
+  f->b = 0;
+  for (int i = 0; i < k; ++i) {
+    const int x = 2 * (n - 1 - hb.wires[k - 1 - i]);
+    f->bit[i] = x;
+    f->bit[k + i] = x + 1;
+    f->col[i] = a.col[i];
+    // column i of A^-T: row i of A^-1
+    f->col[k + i] = 0;
+    for (int o = 0; o < k; ++o) f->col[k + i] |= (inv[o] >> i & 1u) << (k + o);
+  }
+  return true;
+}
+
+// A constant one-qubit superoperator on (ket, bra) that keeps the trace and
+// Hermiticity: a real matrix on Pauli coefficients with first row (1, 0, 0, 0).
+bool pauli_map(const std::vector<cd>& s) {
+  if (s.size() != 16) return false;
+  const cd i1(0, 1);
+  const cd q[4][4] = {{1, 0, 0, 1}, {0, 1, 1, 0}, {1, 0, 0, -1}, {0, -i1, i1, 0}};  // I, X, Z, Y row-major
+  for (int c = 0; c < 4; ++c) {
+    cd x[4];
+    for (int r = 0; r < 4; ++r) {
+      x[r] = 0;
+      for (int t = 0; t < 4; ++t) x[r] += s[4 * r + t] * q[c][t];
+    }
+    if (std::abs(x[0] + x[3] - cd(c == 0 ? 2 : 0, 0)) > 1e-12) return false;
+    if (std::abs((x[1] + x[2]).imag()) > 1e-12 || std::abs((x[0] - x[3]).imag()) > 1e-12 ||
+        std::abs((x[2] - x[1]).real()) > 1e-12)
+      return false;
+  }
+  return true;
+}
+
 bool is_unitary2(const std::vector<cd>& m) {
   if (m.size() != 4) return false;
   for (int i = 0; i < 2; ++i)
@@ -919,11 +969,76 @@ int build_plan(const jq_op* ops, int n_ops, const jq_obs* obs, int n_obs, int n_
     // 20 qubits 3.87 against 3.63 ms.
     const int ft = nb <= kFrameMaxT ? nb : 11;
     const int fc = dtype == JQ_C64 && nb >= 24 ? 4 : 3;
-    if (ok && frame_schedule(fops, nb, ft, fc, dtype == JQ_C64 ? 8 : 16, &zt, &zsign, &plan->frame)) {
+    if (ok && frame_schedule(fops, nb, ft, fc, dtype == JQ_C64 ? 8 : 16, ft == nb ? kFrameMaxStages : kFrameBallot, &zt, &zsign, &plan->frame)) {
       plan->frame_obs = plan->obs;
       for (int i = 0; i < n_obs; ++i) {
         plan->frame_obs[i].z_mask = zt[i];
         plan->frame_obs[i].coeff = obs[i].coeff * zsign[i];
+      }
+    }
+  }
+  // ---- Pauli-basis plan (pauli.cu): Pauli expectation values of a density matrix
+  // under one-qubit gates, one-qubit trace-preserving channels and linear basis
+  // permutations, default tuning, 5 qubits or more (tiles of 10 or 11 bits) ------
+  if (tune && tune->expval_only && mode == JQ_DENSITY && n_obs > 0 && tune->jit == 0 && tune->tile_bits == 0 &&
+      tune->tile_bits_adj == 0 && tune->threads == 0 && tune->ckpt_stride == 0 && !no_fuse && n >= 5) {
+    bool ok = true;
+    for (int i = 0; i < n_obs; ++i) ok = ok && obs[i].kind == JQ_OBS_PAULI;
+    std::vector<FrameOp> fops;
+    for (size_t b = 0; b < blocks.size() && ok; ++b) {
+      const HostBlock& hb = blocks[b];
+      const DevBlock& db = plan->blocks[b];
+      FrameOp f;
+      if (hb.wires.size() == 2 && hb.wires[0] < n && hb.wires[1] == hb.wires[0] + n) {
+        int kind = db.kind == BK_DIAG ? 1 : 0;
+        if (db.kind == BK_PERM) {  // I or X (ket and bra alike)
+          if (hb.st.perm == std::vector<int32_t>{0, 1, 2, 3}) continue;
+          ok = hb.st.perm == std::vector<int32_t>{3, 2, 1, 0};
+          kind = 2;
+        } else {
+          ok = db.n_ctrl == 0;
+        }
+        for (int pi : hb.prims) {
+          const HostPrim& p = prims[pi];
+          if (!ok) break;
+          if (p.form == PF_CONST) { ok = pauli_map(p.cmat); continue; }
+          const int k = p.op >= 0 ? plan->ops[p.op].kind : -1;
+          ok = p.form == PF_KRON && (k == JQ_K_RX || k == JQ_K_RY || k == JQ_K_RZ || k == JQ_K_ROT || k == JQ_K_CPHASE ||
+                                     k == JQ_K_PAULIROT);
+        }
+        f.block = static_cast<int>(b);
+        f.k = 2;
+        f.bit[0] = 2 * (n - 1 - hb.wires[0]);
+        f.bit[1] = f.bit[0] + 1;
+        f.gate = {static_cast<int32_t>(b), db.mat_off < 0 ? 0 : db.mat_off, kind, db.grad_off >= 0 ? 0 : -1, 0, 0};
+      } else {
+        // a permutation of ket wires, then the same one of the bra wires
+        ok = db.kind == BK_PERM && b + 1 < blocks.size() && plan->blocks[b + 1].kind == BK_PERM &&
+             blocks[b + 1].st.perm == hb.st.perm && blocks[b + 1].wires.size() == hb.wires.size();
+        for (size_t i = 0; i < hb.wires.size() && ok; ++i)
+          ok = hb.wires[i] < n && blocks[b + 1].wires[i] == hb.wires[i] + n;
+        ok = ok && pauli_perm(hb, n, &f);
+        ++b;
+      }
+      if (ok) fops.push_back(f);
+    }
+    // Six stages a pass at most (five in float64): the reverse pass keeps every
+    // stage's input tile in shared memory.
+    std::vector<uint64_t> none;
+    std::vector<double> sign;
+    if (ok && frame_schedule(fops, nb, std::min(nb, 11), 3, dtype == JQ_C64 ? 4 : 8,
+                             dtype == JQ_C64 ? 6 : 5, &none, &sign, &plan->pauli)) {
+      for (int i = 0; i < n_obs; ++i) {
+        // physical index of the word: the masks of its x and z bits; stored
+        // coefficients carry (-1)^floor(y / 2)
+        PauliObs o{0u, obs[i].coeff};
+        for (int w = 0; w < n; ++w) {
+          if (obs[i].x_mask >> (n - 1 - w) & 1ULL) o.index ^= plan->pauli.mask[2 * (n - 1 - w)];
+          if (obs[i].z_mask >> (n - 1 - w) & 1ULL) o.index ^= plan->pauli.mask[2 * (n - 1 - w) + 1];
+        }
+        const int y = __builtin_popcountll(obs[i].x_mask & obs[i].z_mask);
+        if (y >> 1 & 1) o.coeff = -o.coeff;
+        plan->pauli_obs.push_back(o);
       }
     }
   }

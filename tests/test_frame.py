@@ -139,3 +139,129 @@ def test_frame_plans_run_fewer_passes():
     plan = _plan(script, (torch.zeros(layers, n, 3),), [jq.PauliZ(0)], n, torch.complex64)
     assert plan.info["n_passes_fwd"] < 2 * layers
     assert plan.info["n_tile_ops_fwd"] == n * layers
+
+
+# ---- noisy circuits on Pauli coefficients (csrc/pauli.cu) --------------------
+def _noisy(n, seed, layers, p):
+    """Rotations, constants and every one-qubit channel on each wire, X, CX and
+    SWAP between them; returns the number of parameters used."""
+    rng = np.random.default_rng(seed)
+    k = 0
+    for _ in range(layers):
+        for w in range(n):
+            kind = int(rng.integers(7))
+            jq.Rot(p[k], p[k + 1], p[k + 2], wires=w)
+            k += 3
+            if kind == 0:
+                jq.DepolarizingChannel(0.03, wires=w)
+            elif kind == 1:
+                jq.AmplitudeDamping(0.05, wires=w)
+            elif kind == 2:
+                jq.RX(p[k], wires=w)
+                k += 1
+                jq.ThermalRelaxationError(0.1, 3.0, 2.0, 0.4, wires=w)
+            elif kind == 3:
+                jq.H(wires=w)
+                jq.BitFlip(0.04, wires=w)
+            elif kind == 4:
+                jq.RZ(p[k], wires=w)
+                k += 1
+                jq.PhaseDamping(0.06, wires=w)
+        for _ in range(n):
+            w, v = (int(x) for x in rng.choice(n, 2, replace=False))
+            kind = int(rng.integers(6))
+            if kind == 0:
+                jq.SWAP(wires=[w, v])
+            elif kind == 1:
+                jq.PauliX(wires=w)
+            else:
+                jq.CX(wires=[w, v])
+            if kind == 2:
+                jq.RZ(p[k], wires=v)  # a diagonal block of its own
+                k += 1
+            elif kind == 3:
+                jq.PhaseFlip(0.05, wires=w)
+    return k
+
+
+def _words(n):
+    y = np.array([[0, -1j], [1j, 0]])
+    z = np.diag([1.0, -1.0])
+    x = np.array([[0, 1.0], [1.0, 0]])
+    return [jq.PauliZ(0), jq.PauliX(n - 1), jq.PauliY(1), jq.build_parity_observable([0, n - 1]),
+            jq.Hermitian(np.kron(y, np.kron(x, y)), wires=[0, 2, 3], record=False),
+            jq.Hermitian(0.5 * np.kron(y, z), wires=[1, n - 1], record=False)]
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("n,layers", [(5, 1), (5, 6), (6, 3)])
+def test_pauli_basis_values_and_gradients(n, layers, dtype):
+    """Values of X, Y, Z and mixed words against the oracle, angle gradients
+    against its central differences."""
+    rng = np.random.default_rng(n + layers)
+    base = rng.uniform(0, 2 * np.pi, 8 * n * layers)
+    base[::4] = rng.integers(0, 5, base[::4].size) * (np.pi / 2)
+    script = jq.Script(lambda p: _noisy(n, 7 * n + layers, layers, p) and None, n_qubits=n)
+    obs = _words(n)
+    ct = rng.normal(size=len(obs))
+    params = torch.tensor(base, requires_grad=True)
+    ev = script.execute("expval", obs, args=(params,), dtype=dtype)
+
+    def reference(b):
+        recs = to_records(script.record(torch.tensor(b)))
+        return O.expval_density(O.simulate_mixed(recs, n), n, obs_records(obs))
+
+    np.testing.assert_allclose(ev.detach().cpu().numpy(), reference(base), atol=TOL[dtype], rtol=0)
+    (ev.to(torch.float64) @ torch.tensor(ct, device=ev.device)).backward()
+    h = 1e-5
+    used = np.flatnonzero(params.grad.numpy())
+    for k in rng.choice(used, 6, replace=False):
+        lo, hi = base.copy(), base.copy()
+        lo[k] -= h
+        hi[k] += h
+        fd = ((reference(hi) - reference(lo)) / (2 * h)) @ ct
+        np.testing.assert_allclose(params.grad[k].item(), fd, atol=TOL[dtype] * n + 1e-8)
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("n,layers,batch", [(6, 2, 5), (7, 3, 3), (9, 2, 1)])
+def test_pauli_basis_against_the_general_passes(n, layers, batch, dtype):
+    """The same circuit with an explicit |0..0> start runs the general passes:
+    values and every gradient, batched; coarse and fine checkpoints alike."""
+    rng = np.random.default_rng(n)
+    base = torch.tensor(rng.uniform(0, 2 * np.pi, (batch, 8 * n * layers)))
+    script = jq.Script(lambda p: _noisy(n, n, layers, p) and None, n_qubits=n)
+    obs = [jq.PauliZ(w) for w in range(n)] + [jq.PauliY(1)]
+    zero = torch.zeros(2**n, dtype=dtype)
+    zero[0] = 1
+    got = []
+    for init in (None, zero):
+        params = base.clone().requires_grad_(True)
+        ev = script.execute("expval", obs, args=(params,), in_axes=(0,), initial_state=init, dtype=dtype)
+        ev.sum().backward()
+        got.append((ev.detach().cpu().numpy(), params.grad.numpy()))
+    np.testing.assert_allclose(got[0][0], got[1][0], atol=TOL[dtype], rtol=0)
+    np.testing.assert_allclose(got[0][1], got[1][1], atol=TOL[dtype] * n, rtol=0)
+
+
+def test_pauli_basis_checkpoint_levels():
+    """A long circuit in a workspace that cannot keep every pass input: the
+    segments recomputed from checkpoints give the gradient of the short form."""
+    from jaqsi_b200 import _lib as lib
+
+    n, layers = 11, 4
+    rng = np.random.default_rng(1)
+    base = torch.tensor(rng.uniform(0, 2 * np.pi, 8 * n * layers))
+    script = jq.Script(lambda p: _noisy(n, 3, layers, p) and None, n_qubits=n)
+    obs = [jq.PauliZ(0), jq.PauliX(4)]
+    params = base.clone().requires_grad_(True)
+    ev = script.execute("expval", obs, args=(params,), dtype=torch.complex64)
+    ev.sum().backward()
+    again = base.clone().requires_grad_(True)
+    zero = torch.zeros(2**n, dtype=torch.complex64)
+    zero[0] = 1
+    ev2 = script.execute("expval", obs, args=(again,), initial_state=zero, dtype=torch.complex64)
+    ev2.sum().backward()
+    assert lib is not None
+    np.testing.assert_allclose(ev.detach().cpu().numpy(), ev2.detach().cpu().numpy(), atol=1e-5, rtol=0)
+    np.testing.assert_allclose(params.grad.numpy(), again.grad.numpy(), atol=1e-5 * n, rtol=0)
