@@ -108,12 +108,20 @@ class _Trace:
     def _idx(self, dev):
         d = self._dev.get(dev)
         if d is None:
-            d = ([(i, torch.tensor(pos, dtype=torch.long, device=dev), torch.tensor(idx, dtype=torch.long))
+            d = ([(i, torch.tensor(pos, dtype=torch.long, device=dev), {"cpu": torch.tensor(idx, dtype=torch.long)})
                   for i, pos, idx in self.parts],
                  torch.tensor(self.cpos, dtype=torch.long, device=dev),
                  torch.tensor(self.cval, dtype=torch.float64, device=dev))
             self._dev[dev] = d
         return d
+
+    @staticmethod
+    def _on(idx, device):
+        """The element indices on an argument's device."""
+        t = idx.get(device)
+        if t is None:
+            t = idx[device] = idx["cpu"].to(device)
+        return t
 
     def angles(self, args, dev, batch=None, in_axes=None):
         """float64 angles on `dev`: [n_angles], or [batch, n_angles] with
@@ -122,14 +130,14 @@ class _Trace:
             return None
         parts, cpos, cval = self._idx(dev)
         if batch is None:
-            if len(parts) == 1 and not self.cpos and len(parts[0][2]) == self.n_angles and self._ordered():
+            if len(parts) == 1 and not self.cpos and len(parts[0][2]["cpu"]) == self.n_angles and self._ordered():
                 i, _, idx = parts[0]
-                return args[i].reshape(-1).index_select(0, idx.to(args[i].device)).to(dev, torch.float64)
+                return args[i].reshape(-1).index_select(0, self._on(idx, args[i].device)).to(dev, torch.float64)
             out = torch.zeros(self.n_angles, dtype=torch.float64, device=dev)
             if self.cpos:
                 out = out.index_copy(0, cpos, cval)
             for i, pos, idx in parts:
-                v = args[i].reshape(-1).index_select(0, idx.to(args[i].device)).to(dev, torch.float64)
+                v = args[i].reshape(-1).index_select(0, self._on(idx, args[i].device)).to(dev, torch.float64)
                 out = out.index_copy(0, pos, v)
             return out
         out = torch.zeros((batch, self.n_angles), dtype=torch.float64, device=dev)
@@ -138,9 +146,9 @@ class _Trace:
         for i, pos, idx in parts:
             a, ax = args[i], in_axes[i]
             if ax is None:
-                v = a.reshape(-1).index_select(0, idx.to(a.device)).to(dev, torch.float64).expand(batch, -1)
+                v = a.reshape(-1).index_select(0, self._on(idx, a.device)).to(dev, torch.float64).expand(batch, -1)
             else:
-                v = a.movedim(ax, 0).reshape(batch, -1).index_select(1, idx.to(a.device)).to(dev, torch.float64)
+                v = a.movedim(ax, 0).reshape(batch, -1).index_select(1, self._on(idx, a.device)).to(dev, torch.float64)
             out = out.index_copy(1, pos, v)
         return out
 
@@ -415,9 +423,18 @@ class Script:
 
     @staticmethod
     def _run_chunked(plan, out_type, batch, angles, mats, init, init_b):
-        """Run in chunks that fit in free device memory (jaqsi/memory.py:169-239)."""
+        """Run in chunks that fit in free device memory (jaqsi/memory.py:169-239).
+
+        Asking the driver for the free memory takes 0.2 to 5 ms, so a call of
+        up to 1 GiB runs whole first and is chunked if an allocation fails
+        (its reverse call then halves its batch by itself)."""
         per = plan.workspace_bytes(1, 2 if not (plan.mode == L.JQ_STATEVECTOR and plan.unitary) else 1)
         per += plan.state_elems * (8 if plan.cdtype == torch.complex64 else 16) * 2
+        if per * batch <= 1 << 30:
+            try:
+                return simulation.run_plan(plan, out_type, batch, angles, mats, init, init_b)
+            except torch.OutOfMemoryError:
+                pass
         free, _ = torch.cuda.mem_get_info()
         chunk = max(1, min(batch, int(0.6 * free // max(per, 1))))
         if chunk >= batch:

@@ -13,6 +13,7 @@ from __future__ import annotations
 import contextlib
 import ctypes
 import gc
+import inspect
 import math
 import threading
 from collections import OrderedDict
@@ -67,7 +68,7 @@ def gc_paused():
 
 
 def _device() -> torch.device:
-    if not torch.cuda.is_available():
+    if not torch.cuda.is_initialized() and not torch.cuda.is_available():
         raise RuntimeError(
             "jaqsi_b200 executes circuits on a CUDA GPU (sm_100a) only; no CUDA device is available"
         )
@@ -593,8 +594,8 @@ class _Execute(torch.autograd.Function):
                 init is not None and ctx.needs_input_grad[6])
         if not any(need):
             return None, None, None, None, None, None, None
-        ga, gm, gi = _ExecuteGrad.apply(ctx.plan, ctx.out_type, ctx.batch, ctx.init_batched, need, angles, mats,
-                                        init, state, g)
+        grad = _grad_launch if _plain((angles, mats, init, state, g)) else _ExecuteGrad.apply
+        ga, gm, gi = grad(ctx.plan, ctx.out_type, ctx.batch, ctx.init_batched, need, angles, mats, init, state, g)
         return (None, None, None, None) + _shape_grads(ctx.init_batched, need, angles, mats, ga, gm, gi)
 
     @staticmethod
@@ -629,6 +630,22 @@ class _Execute(torch.autograd.Function):
                             t_init), None
 
 
+# Function.apply binds its arguments to forward's signature on every call:
+# a stored signature spares it the inspection
+_Execute.forward.__signature__ = inspect.signature(_Execute.forward)
+
+
+def _plain(tensors) -> bool:
+    """Whether a call on these tensors needs no autograd Function: nothing to
+    record (gradients off or not asked for), no torch.func transform around
+    any of them and no forward-mode level open."""
+    grad = torch.is_grad_enabled()
+    for t in tensors:
+        if t is not None and ((grad and t.requires_grad) or _functorch_wrapped(t)):
+            return False
+    return getattr(torch.autograd.forward_ad, "_current_level", 0) < 0
+
+
 def _shape_grads(init_batched, need, angles, mats, ga, gm, gi):
     ga = ga if need[0] else None
     gm = gm if need[1] else None
@@ -643,7 +660,28 @@ def _shape_grads(init_batched, need, angles, mats, ga, gm, gi):
 
 
 def _grad_launch(plan: Plan, out_type: int, batch: int, init_batched: int, need, angles, mats, init, state, g):
-    """Per-instance input gradients [batch, ...] for the output cotangent g."""
+    """Per-instance input gradients [batch, ...] for the output cotangent g;
+    in halves of the batch where the workspace does not fit."""
+    try:
+        return _grad_launch_whole(plan, out_type, batch, init_batched, need, angles, mats, init, state, g)
+    except torch.OutOfMemoryError:
+        if batch < 2:
+            raise
+    cut = batch // 2
+
+    def rows(t, batched, a, b):
+        return t[a:b] if t is not None and batched else t
+
+    parts = []
+    for a, b in ((0, cut), (cut, batch)):
+        parts.append(_grad_launch(
+            plan, out_type, b - a, init_batched, need, rows(angles, angles is not None and angles.dim() == 2, a, b),
+            rows(mats, mats is not None and mats.dim() == 2, a, b), rows(init, init_batched & 1, a, b),
+            state[a:b], g[a:b]))
+    return tuple(torch.cat(p) if p[0].numel() else p[0] for p in zip(*parts))
+
+
+def _grad_launch_whole(plan: Plan, out_type: int, batch: int, init_batched: int, need, angles, mats, init, state, g):
     dev = state.device
     lib = plan._lib
     g = g.contiguous()
@@ -795,7 +833,11 @@ def _jvp_by_rows(plan: Plan, out_type: int, batch: int, init_batched: int, angle
 
 
 def run_plan(plan: Plan, out_type: int, batch: int, angles, mats, init, init_batched: int) -> torch.Tensor:
-    """Execute *plan* for *batch* instances through the autograd Function."""
+    """Execute *plan* for *batch* instances, through the autograd Function
+    where something may be differentiated."""
+    if _plain((angles, mats, init)):
+        state, out = _forward_launch(plan, out_type, batch, init_batched, angles, mats, init)
+        return state if _returns_state(plan, out_type) else out
     return _Execute.apply(plan, out_type, batch, init_batched, angles, mats, init)[0]
 
 
