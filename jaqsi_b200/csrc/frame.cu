@@ -14,54 +14,55 @@
 namespace jq {
 namespace {
 
-// Gate parameters.
-//
-// complex64: U = (phase) Z^z P(f1) [[1, -t], [t, 1]] P(f0) X^piv / norm with
+// Gate parameters: U = (phase) Z^z P(f1) [[1, -t], [t, 1]] P(f0) X^piv / norm with
 // P(f) = diag(1, e^{i f}), |t| <= 1, |f| <= pi / 2.  A phase is three shears,
 // (re, im) -> re - tan(f/2) im, im + sin(f) re, re - tan(f/2) im: five FMA lanes an
-// amplitude and gate, against ten for the 2x2 product.  Rounded shears keep
-// determinant 1; a rounded pair (cos f, sin f) has modulus 1 +- 3e-8, an error
-// that favours one role in every amplitude alike and does not average out (24
-// qubits, 20 layers: 5e-5 of the Z values against 1e-6).  X^piv moves the
-// stage's base address.  Z^z is pushed to the end of the circuit, where it
-// commutes with every Z word: on its way it turns t into -t where the mask
-// crosses its functional (`flip`).  norm is applied every fourth stage.
-//
-// complex128: U = diag(p, q) [[1, -t], [t, 1]] diag(1, u) X^piv.  The phases of a
-// stage's gates are merged into one factor a slot before and after the real
-// rotations: four FP64 operations an amplitude and gate instead of eight.
-struct __align__(16) Gate32 {  // a dense block's row of the block matrices (a diagonal block: its last 16 bytes)
-  float t, tau0, sig0;  // rotation, phase before it (tan(f/2), sin f)
-  uint32_t pad0;
-  float tau1, sig1;     // phase after it
-  uint32_t flags;       // 1: piv, 2: flip
-  uint32_t pad1;
+// amplitude and gate, against ten (complex64, packed) or eight (complex128) for
+// the 2x2 product.  Rounded shears keep determinant 1; a rounded pair (cos f, sin
+// f) has a modulus off by half an ulp, which favours one role in every amplitude
+// alike and does not average out (24 qubits, 20 layers, complex64: 5e-5 of the Z
+// values against 1e-6).  X^piv moves the stage's base address.  Z^z is pushed to
+// the end of the circuit, where it commutes with every Z word: on its way it turns
+// t into -t where the mask crosses its functional (`flip`).  norm is applied every
+// fourth stage.
+template <typename F> struct FlagsOf { using T = uint32_t; };
+template <> struct FlagsOf<double> { using T = uint64_t; };
+// A dense block's row of the block matrices; a diagonal block has the second half.
+template <typename F> struct __align__(16) GateRow {
+  F t, tau0, sig0, pad0;              // rotation; phase before it: tan(f/2), sin f
+  F tau1, sig1;                       // phase after it
+  typename FlagsOf<F>::T flags, pad1; // 1: piv, 2: flip
 };
-static_assert(sizeof(Gate32) == 4 * sizeof(float2), "one 2x2 block");
-__device__ __forceinline__ const Gate32* gate_at(const float2* bm, int off, bool diag) {
-  return reinterpret_cast<const Gate32*>(bm + off - (diag ? 2 : 0));
+static_assert(sizeof(GateRow<float>) == 4 * sizeof(float2) && sizeof(GateRow<double>) == 4 * sizeof(double2),
+              "one 2x2 block");
+template <typename C> struct RealOf;
+template <> struct RealOf<float2> { using T = float; };
+template <> struct RealOf<double2> { using T = double; };
+template <typename C> using Real = typename RealOf<C>::T;
+template <typename C> __device__ __forceinline__ const GateRow<Real<C>>* gate_at(const C* bm, int off, bool diag) {
+  return reinterpret_cast<const GateRow<Real<C>>*>(bm + off - (diag ? 2 : 0));
 }
-__device__ __forceinline__ uint32_t gate_flags(const float2* bm, int off, bool diag) { return gate_at(bm, off, diag)->flags; }
-__device__ __forceinline__ uint32_t gate_flags(const double2* bm, int off, bool diag) {
-  return !diag && bm[off + 3].y != 0.0 ? 1u : 0u;
+template <typename C> __device__ __forceinline__ uint32_t gate_flags(const C* bm, int off, bool diag) {
+  return static_cast<uint32_t>(gate_at(bm, off, diag)->flags);
 }
 
 // Stage tables in shared memory.
-struct __align__(16) Tab32 {
-  float4 g[4];   // t, first phase of the gates (zeros: none)
-  float2 h[4];   // second phase
-  float scale;   // product of 1 / norm over the stages k..  of this group of four
-  uint32_t piv, pad[2];
+template <typename F> struct __align__(16) StageTab {
+  F g[4][4];     // t, first phase of the gates (zeros: none)
+  F h[4][2];     // second phase
+  F scale;       // product of 1 / norm over the stages k.. of k's group of four
+  uint32_t piv;
 };
-struct __align__(16) Tab64 {
-  double2 pre[16], post[16];
-  double t[4];
-  uint32_t piv, pad[3];
-};
-template <typename C> struct TabOf;
-template <> struct TabOf<float2> { using T = Tab32; };
-template <> struct TabOf<double2> { using T = Tab64; };
-template <typename C> using Tab = typename TabOf<C>::T;
+template <typename C> using Tab = StageTab<Real<C>>;
+__device__ __forceinline__ void load_gate(const StageTab<float>& tb, int q, float (&c)[5]) {
+  const float4 g = *reinterpret_cast<const float4*>(tb.g[q]);
+  const float2 h = *reinterpret_cast<const float2*>(tb.h[q]);
+  c[0] = g.x; c[1] = g.y; c[2] = g.z; c[3] = h.x; c[4] = h.y;
+}
+__device__ __forceinline__ void load_gate(const StageTab<double>& tb, int q, double (&c)[5]) {
+  const double2 g = *reinterpret_cast<const double2*>(tb.g[q]), h = *reinterpret_cast<const double2*>(tb.h[q]);
+  c[0] = g.x; c[1] = g.y; c[2] = tb.g[q][2]; c[3] = h.x; c[4] = h.y;
+}
 
 __device__ __forceinline__ void rot_pair(double2& x, double2& y, double t) {
   const double2 a = x;
@@ -76,100 +77,80 @@ __device__ __forceinline__ void rot_pair(float2& x, float2& y, float t) {
   y = __ffma2_rn(make_float2(t, t), a, y);
 }
 // v <- e^{i f} v, tau = tan(f/2), sig = sin f
-__device__ __forceinline__ void shear(float2& v, float tau, float sig) {
-  v.x = fmaf(-tau, v.y, v.x);
-  v.y = fmaf(sig, v.x, v.y);
-  v.x = fmaf(-tau, v.y, v.x);
+template <typename C> __device__ __forceinline__ void shear(C& v, Real<C> tau, Real<C> sig) {
+  v.x = fma(-tau, v.y, v.x);
+  v.y = fma(sig, v.x, v.y);
+  v.x = fma(-tau, v.y, v.x);
 }
 
-// The gates of a stage on 16 slots (slot bit q: role of gate q).
-__device__ __forceinline__ void stage_forward(float2 (&v)[16], const Tab32& tb) {
+// The gates of a stage on 16 slots (slot bit q: role of gate q), and their inverse.
+template <typename C> __device__ __forceinline__ void stage_forward(C (&v)[16], const Tab<C>& tb) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const float4 g = tb.g[q];
-    const float2 h = tb.h[q];
+    Real<C> c[5];
+    load_gate(tb, q, c);
 #pragma unroll
     for (int j = 0; j < 16; ++j)
       if (!(j >> q & 1)) {
         const int m = j | (1 << q);
-        shear(v[m], g.y, g.z);
-        rot_pair(v[j], v[m], g.x);
-        shear(v[m], h.x, h.y);
+        shear(v[m], c[1], c[2]);
+        rot_pair(v[j], v[m], c[0]);
+        shear(v[m], c[3], c[4]);
       }
   }
 }
-__device__ __forceinline__ void stage_forward(double2 (&v)[16], const Tab64& tb) {
-#pragma unroll
-  for (int j = 1; j < 16; ++j) v[j] = cmul(v[j], tb.pre[j]);
+template <typename C> __device__ __forceinline__ void stage_adjoint(C (&v)[16], const Tab<C>& tb) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const double t = tb.t[q];
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (!(j >> q & 1)) rot_pair(v[j], v[j | (1 << q)], t);
-  }
-#pragma unroll
-  for (int j = 0; j < 16; ++j) v[j] = cmul(v[j], tb.post[j]);
-}
-// Their inverse.
-__device__ __forceinline__ void stage_adjoint(float2 (&v)[16], const Tab32& tb) {
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const float4 g = tb.g[q];
-    const float2 h = tb.h[q];
+    Real<C> c[5];
+    load_gate(tb, q, c);
 #pragma unroll
     for (int j = 0; j < 16; ++j)
       if (!(j >> q & 1)) {
         const int m = j | (1 << q);
-        shear(v[m], -h.x, -h.y);
-        rot_pair(v[j], v[m], -g.x);
-        shear(v[m], -g.y, -g.z);
+        shear(v[m], -c[3], -c[4]);
+        rot_pair(v[j], v[m], -c[0]);
+        shear(v[m], -c[1], -c[2]);
       }
   }
 }
-__device__ __forceinline__ void stage_adjoint(double2 (&v)[16], const Tab64& tb) {
-#pragma unroll
-  for (int j = 0; j < 16; ++j) v[j] = cmulc(v[j], tb.post[j]);
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const double t = -tb.t[q];
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (!(j >> q & 1)) rot_pair(v[j], v[j | (1 << q)], t);
-  }
-#pragma unroll
-  for (int j = 1; j < 16; ++j) v[j] = cmulc(v[j], tb.pre[j]);
-}
-// 1 / norm of the stages k.. of k's group of four (complex128: already applied)
-__device__ __forceinline__ float stage_scale(const Tab32& tb) { return tb.scale; }
-__device__ __forceinline__ double stage_scale(const Tab64&) { return 1.0; }
 __device__ __forceinline__ void mul_all(float2 (&v)[16], float f) {
 #pragma unroll
   for (int j = 0; j < 16; ++j) v[j] = __fmul2_rn(v[j], make_float2(f, f));
 }
-__device__ __forceinline__ void mul_all(double2 (&)[16], double) {}
+__device__ __forceinline__ void mul_all(double2 (&v)[16], double f) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    v[j].x *= f;
+    v[j].y *= f;
+  }
+}
 
 // Shared-memory plan of a pass, in bytes.
 template <typename C>
 __host__ __device__ constexpr size_t tab_bytes(int nst) { return static_cast<size_t>(nst) * sizeof(Tab<C>); }
 // Stage tables of one instance.
-template <int LT>
-__device__ __forceinline__ void pass_tables(const FrameStage* __restrict__ st, int nst, const float2* __restrict__ bm, Tab32* tab) {
+template <typename C, int LT>
+__device__ __forceinline__ void pass_tables(const FrameStage* __restrict__ st, int nst, const C* __restrict__ bm, Tab<C>* tab) {
+  using F = Real<C>;
   for (int i = threadIdx.x; i < nst * 8; i += 1 << LT) {
     const FrameStage& s = st[i >> 3];
     const int j = i & 7;
-    Tab32& tb = tab[i >> 3];
+    Tab<C>& tb = tab[i >> 3];
     if (j < 4) {
-      float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
-      float2 h = make_float2(0.f, 0.f);
+      F c[5] = {0, 0, 0, 0, 0};
       if (j < s.ng) {
         const bool diag = s.diag >> (2 * j) & 1;
-        const Gate32* m = gate_at(bm, s.off[j], diag);
-        if (!diag) g = make_float4(m->t, m->tau0, m->sig0, 0.f);
-        h = make_float2(m->tau1, m->sig1);
+        const GateRow<F>* m = gate_at(bm, s.off[j], diag);
+        if (!diag) { c[0] = m->t; c[1] = m->tau0; c[2] = m->sig0; }
+        c[3] = m->tau1;
+        c[4] = m->sig1;
       }
-      tb.g[j] = g;
-      tb.h[j] = h;
+      tb.g[j][0] = c[0];
+      tb.g[j][1] = c[1];
+      tb.g[j][2] = c[2];
+      tb.h[j][0] = c[3];
+      tb.h[j][1] = c[4];
     } else if (j == 4) {
       uint32_t piv = 0;
       for (int q = 0; q < s.ng; ++q) piv |= (gate_flags(bm, s.off[q], s.diag >> (2 * q) & 1) & 1u) << q;
@@ -183,31 +164,7 @@ __device__ __forceinline__ void pass_tables(const FrameStage* __restrict__ st, i
             const double t = gate_at(bm, st[x].off[q], false)->t;  // the rounded one: exactly its norm
             f *= 1.0 + t * t;
           }
-      tb.scale = static_cast<float>(1.0 / sqrt(f));
-    }
-  }
-}
-// float64 products of the gates' phases, rounded once
-template <int LT>
-__device__ __forceinline__ void pass_tables(const FrameStage* __restrict__ st, int nst, const double2* __restrict__ bm, Tab64* tab) {
-  for (int i = threadIdx.x; i < nst * 16; i += 1 << LT) {
-    const FrameStage& s = st[i >> 4];
-    const int j = i & 15;
-    double2 pre = make_double2(1, 0), post = make_double2(1, 0);
-    for (int q = 0; q < s.ng; ++q) {
-      const double2* m = bm + s.off[q];
-      const bool hi = j >> q & 1, diag = s.diag >> (2 * q) & 1;
-      post = cmul(post, m[hi ? 1 : 0]);
-      if (!diag && hi) pre = cmul(pre, m[2]);
-    }
-    Tab64& tb = tab[i >> 4];
-    tb.pre[j] = pre;
-    tb.post[j] = post;
-    if (j < 4) tb.t[j] = (j < s.ng && !(s.diag >> (2 * j) & 1)) ? bm[s.off[j] + 3].x : 0.0;
-    if (j == 4) {
-      uint32_t piv = 0;
-      for (int q = 0; q < s.ng; ++q) piv |= gate_flags(bm, s.off[q], s.diag >> (2 * q) & 1) << q;
-      tb.piv = piv;
+      tb.scale = static_cast<F>(1.0 / sqrt(f));
     }
   }
 }
@@ -268,7 +225,7 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
     // bit 4 k + q: gate q of stage k has its roles exchanged in this tile
     const uint32_t flips = __ballot_sync(0xffffffffu, ((__popc(rep & r_lane) & 1u) ^ s_lane) != 0u);
     if (inst != last) {
-      pass_tables<LT>(st, nst, bmat + inst * bstride, tab);
+      pass_tables<C, LT>(st, nst, bmat + inst * bstride, tab);
       last = inst;
     }
     cp_wait<1>();
@@ -287,8 +244,8 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
       for (int j = 0; j < 16; ++j) v[j] = lds<C>(a[j]);
       // group scale: the table entry of the group's first stage
       const bool rescale = (k & 3) == 3 || k + 1 == nst;
-      stage_forward(v, tb);
-      if (rescale) mul_all(v, stage_scale(tab[k & ~3]));
+      stage_forward<C>(v, tb);
+      if (rescale) mul_all(v, tab[k & ~3].scale);
       if (P.direct && k + 1 == nst) {
         const uint32_t ge[4] = {st[k].ge[0], st[k].ge[1], st[k].ge[2], st[k].ge[3]};
         slot_offsets(ge, rep ^ gout ^ slot_xor(ge, nib), a);
@@ -372,7 +329,7 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
         __syncthreads();
         for (int i = tid; i < NW * nst * 16; i += NT) sacc[i] = 0.0;
       }
-      pass_tables<LT>(st, nst, bmat + inst * bstride, tab);
+      pass_tables<C, LT>(st, nst, bmat + inst * bstride, tab);
       last = inst;
     }
     cp_wait<0>();
@@ -389,12 +346,12 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
         slot_offsets(e, base ^ so[nib], a);
 #pragma unroll
         for (int j = 0; j < 16; ++j) p[j] = lds<C>(a[j]);
-        stage_adjoint(p, tb);
+        stage_adjoint<C>(p, tb);
 #pragma unroll
         for (int j = 0; j < 16; ++j) l[j] = lds<C>(a[j] ^ TB);
-        stage_adjoint(l, tb);
+        stage_adjoint<C>(l, tb);
       }
-      F cs = stage_scale(tb);  // norm of psi and lambda so far in this group
+      F cs = tb.scale;  // norm of psi and lambda so far in this group
       if ((k & 3) == 0) {
         mul_all(p, cs);
         mul_all(l, cs);
@@ -473,36 +430,17 @@ __device__ void block_matrix(const DevBlock& blk, const DevPrim* prims, const De
   }
 }
 
-// Parameters of a complex128 gate (and its Z flag, unused there).
-__device__ uint32_t put_gate(const double2* u, bool diag, double2* out) {
-  if (diag) {
-    out[0] = u[0];
-    out[1] = u[3];
-    return 0;
-  }
-  double2 a = u[0], c = u[2], d = u[3];
-  const double na = a.x * a.x + a.y * a.y, nc = c.x * c.x + c.y * c.y;
-  const bool piv = nc > na;
-  if (piv) { a = u[1]; c = u[3]; d = u[2]; }
-  const double ra = sqrt(piv ? nc : na), rc = sqrt(piv ? na : nc);
-  const double2 ph = rc > 0.0 ? make_double2(c.x / rc, c.y / rc) : make_double2(1.0, 0.0);
-  const double2 q = make_double2(ra * ph.x, ra * ph.y), dq = cmulc(d, q);
-  const double q2 = q.x * q.x + q.y * q.y;
-  out[0] = a;
-  out[1] = q;
-  out[2] = make_double2(dq.x / q2, dq.y / q2);
-  out[3] = make_double2(rc / ra, piv ? 1.0 : 0.0);
-  return 0;
-}
 // tan(f/2), sin f of w / |w| = e^{i f} for Re w >= 0, of -w otherwise (returns 1)
-__device__ uint32_t put_phase(double2 w, float* tau, float* sig) {
+template <typename F> __device__ uint32_t put_phase(double2 w, F* tau, F* sig) {
   const double s = w.x < 0.0 ? -1.0 : 1.0, m = sqrt(w.x * w.x + w.y * w.y);
-  *tau = static_cast<float>(s * w.y / (m + s * w.x));
-  *sig = static_cast<float>(s * w.y / m);
+  *tau = static_cast<F>(s * w.y / (m + s * w.x));
+  *sig = static_cast<F>(s * w.y / m);
   return w.x < 0.0;
 }
-__device__ uint32_t put_gate(const double2* u, bool diag, float2* out) {
-  Gate32* o = reinterpret_cast<Gate32*>(out - (diag ? 2 : 0));
+// Parameters of a gate; returns its Z flag.
+template <typename C> __device__ uint32_t put_gate(const double2* u, bool diag, C* out) {
+  using F = Real<C>;
+  GateRow<F>* o = reinterpret_cast<GateRow<F>*>(out - (diag ? 2 : 0));
   double2 a = u[0], b = u[1], c = u[2], d = u[3];
   uint32_t flags = 0, z = 0;
   if (diag) {
@@ -518,14 +456,14 @@ __device__ uint32_t put_gate(const double2* u, bool diag, float2* out) {
     const double2 e1 = mc > 0.0 ? make_double2(w1.x / mc, w1.y / mc) : make_double2(1.0, 0.0);
     const uint32_t z0 = put_phase(cmulc(w, e1), &o->tau0, &o->sig0);
     z = z0 ^ put_phase(e1, &o->tau1, &o->sig1);
-    const float t = static_cast<float>(mc / a2);
+    const F t = static_cast<F>(mc / a2);
     o->t = z0 ? -t : t;
   }
   o->flags = flags;
   return z;
 }
-__device__ __forceinline__ void put_flip(float2* out, bool diag) {
-  Gate32* o = reinterpret_cast<Gate32*>(out - (diag ? 2 : 0));
+template <typename C> __device__ __forceinline__ void put_flip(C* out, bool diag) {
+  GateRow<Real<C>>* o = reinterpret_cast<GateRow<Real<C>>*>(out - (diag ? 2 : 0));
   o->flags |= 2u;
   if (!diag) o->t = -o->t;
 }
@@ -554,7 +492,7 @@ __global__ void __launch_bounds__(kPrepThreads)
       block_matrix(blocks[fg.block], prims, ops, ang, cpool, u);
       if (put_gate(u, fg.diag, bm + fg.mat_off)) x = fg.r;
     }
-    if constexpr (sizeof(C) == sizeof(float2)) {
+    {
       uint32_t s = x;  // inclusive prefix XOR
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
