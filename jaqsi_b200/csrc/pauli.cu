@@ -34,20 +34,26 @@ __device__ __forceinline__ double flip_sign(double v, uint32_t s) {
 // parity of the number of Y factors
 __device__ __forceinline__ uint32_t y_parity(uint32_t g) { return __popc(g & (g >> 1) & 0x55555555u) & 1u; }
 
-// Which of a thread's 16 slots (slot = wire a + 4 wire b) change sign; g0: index
-// of slot 0, ge: register vectors.
-__device__ __forceinline__ uint32_t slot_signs(uint32_t g0, const FrameStage& st) {
-  const uint32_t p = y_parity(g0);
-  if (st.ng == 2) return (p ? 0x7888u : 0u) | 0x8000u;
-  // one wire: the other register bits are not a wire's
-  return (p << 3) | (y_parity(g0 ^ st.ge[2]) << 7) | (y_parity(g0 ^ st.ge[3]) << 11) |
-         (y_parity(g0 ^ st.ge[2] ^ st.ge[3]) << 15);
+// Signs.  In a stage of two wires slot (a, b) = a + 4 b carries (-1)^(p [a = Y] + p
+// [b = Y] + [a = Y][b = Y]), p the y parity of slot 0.  To a wire's matrix that
+// is one sign on its entries with exactly one Y: (-1)^p, and the other one
+// where the other wire is Y, so the five entries change sign (flip_odd) and the
+// values need none: 10 instead of 28 sign operations on 16 values.
+template <typename F> __device__ __forceinline__ void flip_odd(F (&c)[12], uint32_t p) {
+  c[3] = flip_sign(c[3], p);
+  c[7] = flip_sign(c[7], p);
+  c[8] = flip_sign(c[8], p);
+  c[9] = flip_sign(c[9], p);
+  c[10] = flip_sign(c[10], p);
 }
-template <typename F> __device__ __forceinline__ void apply_signs(F (&v)[16], uint32_t s) {
-  v[3] = flip_sign(v[3], s >> 3 & 1u);
-  v[7] = flip_sign(v[7], s >> 7 & 1u);
-#pragma unroll
-  for (int j = 11; j < 16; ++j) v[j] = flip_sign(v[j], s >> j & 1u);
+__device__ __host__ constexpr bool odd_entry(int e) { return e == 3 || (e >= 7 && e <= 10); }
+// A stage of one wire: its register vectors 2 and 3 are not a wire's, and each of
+// the four columns has its own parity.
+template <typename F> __device__ __forceinline__ void column_signs(F (&v)[16], uint32_t g0, const FrameStage& st) {
+  v[3] = flip_sign(v[3], y_parity(g0));
+  v[7] = flip_sign(v[7], y_parity(g0 ^ st.ge[2]));
+  v[11] = flip_sign(v[11], y_parity(g0 ^ st.ge[3]));
+  v[15] = flip_sign(v[15], y_parity(g0 ^ st.ge[2] ^ st.ge[3]));
 }
 
 // The 12 entries of a wire's matrix, by 16-byte loads.
@@ -66,12 +72,14 @@ __device__ __forceinline__ void load12(const double* m, double (&c)[12]) {
   }
 }
 
-// v <- M v on wire a (S = 1) or b (S = 4)
-template <int S, typename F> __device__ __forceinline__ void apply_m(F (&v)[16], const F* m) {
-  F c[12];
-  load12(m, c);
+// v <- M v on wire a (S = 1) or b (S = 4); PAIR: the other wire's Y (group 3)
+// takes the odd entries with the other sign
+template <int S, bool PAIR, typename F> __device__ __forceinline__ void apply_m(F (&v)[16], const F (&m)[12]) {
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
+    F c[12];
+#pragma unroll
+    for (int e = 0; e < 12; ++e) c[e] = PAIR && g == 3 && odd_entry(e) ? -m[e] : m[e];
     const int b = S == 1 ? 4 * g : g;
     const F a0 = v[b], a1 = v[b + S], a2 = v[b + 2 * S], a3 = v[b + 3 * S];
 #pragma unroll
@@ -80,11 +88,12 @@ template <int S, typename F> __device__ __forceinline__ void apply_m(F (&v)[16],
   }
 }
 // v <- M^T v
-template <int S, typename F> __device__ __forceinline__ void apply_mt(F (&v)[16], const F* m) {
-  F c[12];
-  load12(m, c);
+template <int S, bool PAIR, typename F> __device__ __forceinline__ void apply_mt(F (&v)[16], const F (&m)[12]) {
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
+    F c[12];
+#pragma unroll
+    for (int e = 0; e < 12; ++e) c[e] = PAIR && g == 3 && odd_entry(e) ? -m[e] : m[e];
     const int b = S == 1 ? 4 * g : g;
     const F a1 = v[b + S], a2 = v[b + 2 * S], a3 = v[b + 3 * S];
     v[b] = fma(c[8], a3, fma(c[4], a2, fma(c[0], a1, v[b])));
@@ -93,7 +102,8 @@ template <int S, typename F> __device__ __forceinline__ void apply_mt(F (&v)[16]
   }
 }
 // g[4 (i - 1) + j] = sum of l (entry i of the wire) times x (entry j), i = 1..3
-template <int S, typename F> __device__ __forceinline__ void outer_sum(const F (&l)[16], const F (&x)[16], F (&g)[16]) {
+template <int S, bool PAIR, typename F>
+__device__ __forceinline__ void outer_sum(const F (&l)[16], const F (&x)[16], F (&g)[16]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -102,12 +112,36 @@ template <int S, typename F> __device__ __forceinline__ void outer_sum(const F (
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int b = S == 1 ? 4 * q : q;
-        a = fma(l[b + (i + 1) * S], x[b + j * S], a);
+        const F y = x[b + j * S];
+        a = fma(l[b + (i + 1) * S], PAIR && q == 3 && odd_entry(4 * i + j) ? -y : y, a);
       }
       g[4 * i + j] = a;
     }
 #pragma unroll
   for (int i = 12; i < 16; ++i) g[i] = 0;
+}
+template <typename F> __device__ __forceinline__ void flip_sums(F (&g)[16], uint32_t p) {
+#pragma unroll
+  for (int e = 0; e < 12; ++e)
+    if (odd_entry(e)) g[e] = flip_sign(g[e], p);
+}
+// A stage's matrices on its 16 values.
+template <typename F>
+__device__ __forceinline__ void stage_values(F (&v)[16], const PTab<F>& tb, uint32_t g0, const FrameStage& st) {
+  F c[12];
+  load12(tb.m[0], c);
+  if (st.ng == 2) {
+    const uint32_t p = y_parity(g0);
+    flip_odd(c, p);
+    apply_m<1, true>(v, c);
+    load12(tb.m[1], c);
+    flip_odd(c, p);
+    apply_m<4, true>(v, c);
+  } else {
+    column_signs(v, g0, st);
+    apply_m<1, false>(v, c);
+    column_signs(v, g0, st);
+  }
 }
 
 template <typename F, int LT>
@@ -148,11 +182,13 @@ template <typename F> __host__ __device__ constexpr size_t pauli_tables(int nst,
 }
 
 // One forward pass, `in` to `out` (the same buffer: in place).  Bound by
-// instruction issue (60 to 75% of its slots; 14 to 17 instructions a value and
-// stage, 6 of them FMAs) with DRAM at 30%.  12 qubits, 8 layers, complex64, value
-// and gradient: 19.3 -> 7.1 ms a call (32 passes of 75 us each way against 61 of
-// 110 us and reverse steps of 200 us on matrix entries); 7 qubits, 5 layers,
-// complex128, 16 sets: 4.1 -> 0.8 ms.
+// instruction issue (51 to 65% of its slots; 18 instructions a value and stage, 6
+// of them FMAs) and shared-memory wavefronts (18 stages of 107 conflict) with DRAM
+// at 30 to 40%.  12 qubits, 8 layers, complex64, value and gradient: 19.3 -> 6.7 ms
+// a call (32 passes of 47 to 56 us forward, twice, and of 105 us back, against 61
+// of 110 us and reverse steps of 200 us on matrix entries); 7 qubits, 5 layers,
+// complex128, 16 sets: 3.9 -> 0.45 ms.  Signs in the matrices instead of on the
+// values and the first tables formed before the wait: 6.94 -> 6.72 ms.
 template <typename F, int T, int MINB>
 __global__ void __launch_bounds__(1 << (T - 4), MINB)
     k_pauli_fwd(const F* in, F* out, const PassArg P, const FrameStage* __restrict__ stages, const F* __restrict__ bmat,
@@ -184,11 +220,16 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
     const F* src = in + ((tl >> P.nouter) << P.nb);
     copy.each(P, rep_of(tl), dst, [&](uint32_t a, uint32_t b) { cp_async16(sbase + b, src + a); });
   };
+  // k_pauli_init has run since prep: the matrices need no wait, the states do
+  int64_t last = -1;
+  if (blockIdx.x < ntiles) {
+    last = static_cast<int64_t>(blockIdx.x) >> P.nouter;
+    pass_tables<F, LT>(st, nst, bmat + last * bstride, tab);
+  }
   __syncthreads();
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (blockIdx.x < ntiles) load(0, blockIdx.x);
   cp_commit();
-  int64_t last = -1;
   uint32_t s = 0;
   for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     if (tile + gridDim.x < ntiles) load(s ^ TB, tile + gridDim.x);
@@ -204,7 +245,6 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
     __syncthreads();
     F* g = out + (inst << P.nb);
     for (int k = 0; k < nst; ++k) {
-      const PTab<F>& tb = tab[k];
       const uint32_t nib = (flips >> (4 * k)) & 15u;
       const uint32_t* so = soff + 16 * k;
       const uint32_t e[4] = {so[1], so[2], so[4], so[8]};
@@ -215,11 +255,7 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
       slot_offsets(e, base, a);
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] = lds<F>(a[j]);
-      const uint32_t sg = slot_signs(g0, st[k]);
-      apply_signs(v, sg);
-      apply_m<1>(v, tb.m[0]);
-      apply_m<4>(v, tb.m[1]);
-      apply_signs(v, sg);
+      stage_values(v, tab[k], g0, st[k]);
       if (P.direct && k + 1 == nst) {
         const uint32_t ge[4] = {gso[16 * k + 1], gso[16 * k + 2], gso[16 * k + 4], gso[16 * k + 8]};
         slot_offsets(ge, g0, a);
@@ -243,6 +279,8 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
 // after its matrix times entries of the values before it, the other wire's matrix
 // on one side) is summed, per tile and warp in the run precision, in float64
 // across tiles, and lambda goes through the transposed matrices.
+// Not launched ahead of the previous pass: two of these on an SM at once take each
+// other's L2 (12 qubits 7.08 instead of 6.72 ms).
 template <typename F, int T, int MINB>
 __global__ void __launch_bounds__(1 << (T - 4), MINB)
     k_pauli_bwd(const F* __restrict__ xin, F* __restrict__ lam, const PassArg P, const FrameStage* __restrict__ stages,
@@ -309,14 +347,11 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
     };
     for (int k = 0; k + 1 < nst; ++k) {
       uint32_t a[16];
-      const uint32_t sg = slot_signs(slots(k, a), st[k]);
+      const uint32_t g0 = slots(k, a);
       F v[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] = lds<F>(k * TB + a[j]);
-      apply_signs(v, sg);
-      apply_m<1>(v, tab[k].m[0]);
-      apply_m<4>(v, tab[k].m[1]);
-      apply_signs(v, sg);
+      stage_values(v, tab[k], g0, st[k]);
 #pragma unroll
       for (int j = 0; j < 16; ++j) sts(k * TB + TB + a[j], v[j]);
       __syncthreads();
@@ -325,37 +360,57 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
       const PTab<F>& tb = tab[k];
       uint32_t a[16];
       const uint32_t g0 = slots(k, a);
-      const uint32_t sg = slot_signs(g0, st[k]);
-      F l[16];
+      F l[16], c[12];
 #pragma unroll
       for (int j = 0; j < 16; ++j) l[j] = lds<F>(lt + a[j]);
-      apply_signs(l, sg);
       double* acc = sacc + (warp * nst + k) * 32;
       const bool wa = gacc && st[k].gate[0] >= 0, wb = gacc && st[k].ng > 1 && st[k].gate[2] >= 0;
+      auto add = [&](double* to, F (&g)[16]) {
+        const F t = warp_rs16(g, lane);
+        if (!(lane & 1u)) to[lane >> 1] += static_cast<double>(t);
+      };
       F x[16];
       if (wa || wb) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) x[j] = lds<F>(k * TB + a[j]);
-        apply_signs(x, sg);
       }
-      if (wb) {
-        F y[16], g[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) y[j] = x[j];
-        apply_m<1>(y, tb.m[0]);
-        outer_sum<4>(l, y, g);
-        const F t = warp_rs16(g, lane);
-        if (!(lane & 1u)) acc[16 + (lane >> 1)] += static_cast<double>(t);
-      }
-      apply_mt<4>(l, tb.m[1]);
-      if (wa) {
+      if (st[k].ng == 2) {
+        const uint32_t p = y_parity(g0);
         F g[16];
-        outer_sum<1>(l, x, g);
-        const F t = warp_rs16(g, lane);
-        if (!(lane & 1u)) acc[lane >> 1] += static_cast<double>(t);
+        if (wb) {
+          F y[16];
+          load12(tb.m[0], c);
+          flip_odd(c, p);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) y[j] = x[j];
+          apply_m<1, true>(y, c);
+          outer_sum<4, true>(l, y, g);
+          flip_sums(g, p);
+          add(acc + 16, g);
+        }
+        load12(tb.m[1], c);
+        flip_odd(c, p);
+        apply_mt<4, true>(l, c);
+        if (wa) {
+          outer_sum<1, true>(l, x, g);
+          flip_sums(g, p);
+          add(acc, g);
+        }
+        load12(tb.m[0], c);
+        flip_odd(c, p);
+        apply_mt<1, true>(l, c);
+      } else {
+        column_signs(l, g0, st[k]);
+        if (wa) {
+          F g[16];
+          column_signs(x, g0, st[k]);
+          outer_sum<1, false>(l, x, g);
+          add(acc, g);
+        }
+        load12(tb.m[0], c);
+        apply_mt<1, false>(l, c);
+        column_signs(l, g0, st[k]);
       }
-      apply_mt<1>(l, tb.m[0]);
-      apply_signs(l, sg);
 #pragma unroll
       for (int j = 0; j < 16; ++j) sts(lt + a[j], l[j]);
       __syncthreads();
