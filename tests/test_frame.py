@@ -265,3 +265,36 @@ def test_pauli_basis_checkpoint_levels():
     assert lib is not None
     np.testing.assert_allclose(ev.detach().cpu().numpy(), ev2.detach().cpu().numpy(), atol=1e-5, rtol=0)
     np.testing.assert_allclose(params.grad.numpy(), again.grad.numpy(), atol=1e-5 * n, rtol=0)
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("n", [9, 10, 11, 12, 13])
+@pytest.mark.parametrize("frame", [True, False])
+def test_seed_of_many_z_strings(n, frame, dtype):
+    """The reverse pass's seed over Z strings: the smallest sizes of both thread
+    widths, more words than one load holds, zero cotangents, and an instance
+    whose cotangents are all zero."""
+    gates, rng = 30, np.random.default_rng(100 + n)
+    inner = _circuit(n, 7 * n, gates)
+
+    def body(p):
+        if not frame:
+            jq.CRX(p[-1], wires=[0, n - 1])
+        inner(p)
+
+    base = rng.uniform(0, 2 * np.pi, (2, 3 * gates + 4))
+    obs = [jq.PauliZ(w) for w in range(n)]
+    obs += [jq.build_parity_observable([a, b]) for a in range(n) for b in range(a + 1, n)]
+    ct = rng.normal(size=(2, len(obs)))
+    ct[0, ::3] = 0.0
+    ct[1] = 0.0
+    script = jq.Script(lambda p: body(p) and None, n_qubits=n)
+    params = torch.tensor(base, requires_grad=True)
+    ev = script.execute("expval", obs, args=(params,), in_axes=(0,), dtype=dtype)
+    (ev.to(torch.float64) * torch.tensor(ct, device=ev.device)).sum().backward()
+    _, ref = O.adjoint_grad(to_records(script.record(torch.tensor(base[0]))), n, obs_records(obs), ct=ct[0])
+    got = params.grad[0].numpy()
+    if not frame:  # recorded first, held last
+        got = np.concatenate([got[-1:], got[:-1]])
+    np.testing.assert_allclose(got[: len(ref)], ref, atol=TOL[dtype] * np.abs(ct[0]).sum(), rtol=0)
+    assert not params.grad[1].any()
