@@ -148,18 +148,22 @@ typedef struct jq_tune {
                             and not run; the state buffers then hold the
                             state before them (jq_sweep applies the passes
                             the plan keeps), and other out types fail with
-                            JQ_EINVAL.  A plan of one-wire unitaries and
-                            affine permutations only (default tile sizes,
-                            jit 0, 9 qubits or more) moves no amplitude for
-                            any permutation: its state buffers hold the
-                            amplitudes at linearly mapped indices, up to
-                            signs, for jq_adjoint of the same plan.  A density
-                            plan of one-qubit gates, one-qubit channels and
-                            X / CX / SWAP-like permutations with Pauli words
-                            (default tuning, 5 qubits or more) runs
-                            expectation values from |0..0> (init NULL) on
-                            Pauli coefficients; the state buffer then holds
-                            those.                                             */
+                            JQ_EINVAL.  2: as 1, and what the state buffers
+                            hold is the plan's own affair, to be passed on to
+                            jq_adjoint / jq_sweep of the same plan only.  A
+                            plan of one-wire unitaries and affine permutations
+                            (default tile sizes, jit 0, 9 qubits or more) then
+                            moves no amplitude for any permutation: its
+                            buffers hold the amplitudes at linearly mapped
+                            indices, up to signs.  A density plan of one-qubit
+                            gates, one-qubit channels and X / CX / SWAP-like
+                            permutations with Pauli words (default tuning, 5
+                            qubits or more) runs expectation values from
+                            |0..0> (init NULL) on Pauli coefficients.  Calls
+                            for another out type (where nothing was absorbed)
+                            and jq_backward of a statevector plan run the
+                            circuit itself, on amplitudes at their own
+                            indices.                                           */
 } jq_tune;
 
 /* Plan summary. */

@@ -2130,7 +2130,7 @@ int upload(const std::vector<T>& v, T** dst) {
 // The plan's NVRTC specialisation on the current device.
 void build_jit(const jq_plan* plan, DeviceTables* t) {
   t->jit_tried = true;
-  if (plan->jit && !plan->frame.on && jit_available()) {
+  if (plan->jit && jit_available()) {
     JitModule* jm = new JitModule();
     const int rc = jit_build(plan, plan->fwd, jm);
     if (rc == JQ_OK) {
@@ -2151,16 +2151,23 @@ void build_jit(const jq_plan* plan, DeviceTables* t) {
   }
 }
 
-// general: the call runs the general passes (a Pauli-basis plan compiles their
-// specialisation on the first such call only)
-int device_tables(const jq_plan* cplan, const DeviceTables** out, bool general = true) {
+// Set while a call must not allocate device memory (jq_forward_noalloc).
+thread_local bool tl_no_build = false;
+
+// general: the call runs the general passes.  A frame or Pauli-basis plan
+// compiles their specialisation on the first such call only, not within a
+// capture of st or a call that may not allocate (those interpret the schedule).
+int device_tables(const jq_plan* cplan, const DeviceTables** out, bool general = true, cudaStream_t st = nullptr) {
   jq_plan* plan = const_cast<jq_plan*>(cplan);
   int dev = 0;
   JQ_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lock(g_upload_mu);
   for (DeviceTables& t : plan->dev)
     if (t.device == dev) {
-      if (general && !t.jit_tried) build_jit(plan, &t);
+      if (general && !t.jit_tried && !tl_no_build) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) build_jit(plan, &t);
+      }
       if (t.jit_rc) {
         set_error(t.jit_err);
         return t.jit_rc;
@@ -2189,7 +2196,7 @@ int device_tables(const jq_plan* cplan, const DeviceTables** out, bool general =
   if ((rc = upload(plan->fwd.rops, &t.fwd_rops))) return rc;
   if ((rc = upload(plan->bwd.steps, &t.bwd_steps))) return rc;
   if ((rc = upload(plan->bwd.rops, &t.bwd_rops))) return rc;
-  if (general || !plan->pauli.on) build_jit(plan, &t);
+  if (general || !(plan->pauli.on || plan->frame.on)) build_jit(plan, &t);
   if (plan->frame.on) {
     if ((rc = frame_upload(plan, &t.frame))) return rc;
     DevObs* fo = nullptr;
@@ -2314,7 +2321,6 @@ int run_passes(const jq_plan* plan, const Schedule& sch, const TileOp* dops, con
                const RegOp* drops, const DeviceTables* T, typename CplxT<R>::T* state, int batch,
                const typename CplxT<R>::T* bmat, size_t p0, size_t p1, cudaStream_t st,
                const JitModule* jm = nullptr) {
-  if (plan->frame.on) return frame_forward(plan, T->frame, state, batch, bmat, sm_count(), st);
   constexpr int RB = 4;
   for (size_t p = p0; p < p1; ++p) {
     const PassDesc& pd = sch.passes[p];
@@ -2350,10 +2356,10 @@ int run_passes(const jq_plan* plan, const Schedule& sch, const TileOp* dops, con
 
 template <typename R>
 int prep(const jq_plan* plan, const DeviceTables* T, int batch, const double* angles, const void* mats,
-         typename CplxT<R>::T* bmat, double2* scratch, cudaStream_t st) {
+         typename CplxT<R>::T* bmat, double2* scratch, cudaStream_t st, bool frame = false) {
   const int nbk = static_cast<int>(plan->blocks.size());
   if (nbk == 0) return JQ_OK;
-  if (plan->frame.on)
+  if (frame)
     return frame_prep(plan, T->frame, T->blocks, T->prims, T->ops, T->const_pool, batch, angles, bmat, st);
   const int64_t work = static_cast<int64_t>(nbk) * batch;
   const int threads = 128;
@@ -2368,7 +2374,7 @@ int prep(const jq_plan* plan, const DeviceTables* T, int batch, const double* an
 
 template <typename R>
 int measure(const jq_plan* plan, const DeviceTables* T, int batch, int out_type, const typename CplxT<R>::T* state,
-            void* out, cudaStream_t st) {
+            void* out, cudaStream_t st, bool frame = false) {
   using C = typename CplxT<R>::T;
   const int n = plan->n_qubits;
   const int64_t dim = 1LL << n;
@@ -2389,8 +2395,8 @@ int measure(const jq_plan* plan, const DeviceTables* T, int batch, int out_type,
     if (n_obs == 0) return JQ_OK;
     double* o = static_cast<double*>(out);
     JQ_CUDA(cudaMemsetAsync(o, 0, sizeof(double) * n_obs * batch, st));
-    const std::vector<DevObs>& pobs = plan->frame.on ? plan->frame_obs : plan->obs;
-    const DevObs* od = static_cast<const DevObs*>(plan->frame.on ? T->frame_obs : T->obs_desc);
+    const std::vector<DevObs>& pobs = frame ? plan->frame_obs : plan->obs;
+    const DevObs* od = static_cast<const DevObs*>(frame ? T->frame_obs : T->obs_desc);
     const double2* pool = reinterpret_cast<const double2*>(T->obs_pool);
     // Pauli observables in chunks; dense ones one launch each
     int i = 0;
@@ -2450,14 +2456,18 @@ bool pauli_call(const jq_plan* plan, int out_type, const void* init) {
   return plan->pauli.on && out_type == JQ_OUT_EXPVAL && !init;
 }
 
+// Whether a call of a frame plan runs in its frame: expectation values and their
+// gradients by the adjoint; anything else is the circuit itself.
+bool frame_call(const jq_plan* plan, int out_type) { return plan->frame.on && out_type == JQ_OUT_EXPVAL; }
+
 template <typename R>
 int forward_impl(const jq_plan* plan, int batch, const double* angles, const void* mats, const void* init,
                  int init_batched, int out_type, void* state, void* out, void* ws, size_t ws_bytes,
                  cudaStream_t st) {
   using C = typename CplxT<R>::T;
   const DeviceTables* T = nullptr;
-  const bool pauli = pauli_call(plan, out_type, init);
-  int rc = device_tables(plan, &T, !pauli);
+  const bool pauli = pauli_call(plan, out_type, init), frame = frame_call(plan, out_type);
+  int rc = device_tables(plan, &T, !pauli && !frame, st);
   if (rc) return rc;
   if ((rc = set_smem_attrs<R>())) return rc;
   WsLayout L = layout(plan, batch, 0);
@@ -2469,7 +2479,7 @@ int forward_impl(const jq_plan* plan, int batch, const double* angles, const voi
   C* bmat = reinterpret_cast<C*>(w + L.bmat);
   if (pauli) return pauli_forward(plan, *T, batch, angles, state, bmat, static_cast<double*>(out), sm_count(), st);
   double2* scratch = reinterpret_cast<double2*>(w + L.scratch);
-  if ((rc = prep<R>(plan, T, batch, angles, mats, bmat, scratch, st))) return rc;
+  if ((rc = prep<R>(plan, T, batch, angles, mats, bmat, scratch, st, frame))) return rc;
   C* S = static_cast<C*>(state);
   const bool dm = plan->mode == JQ_DENSITY;
   const int64_t dim = 1LL << plan->n_qubits;
@@ -2478,6 +2488,10 @@ int forward_impl(const jq_plan* plan, int batch, const double* angles, const voi
       S, plan->state_elems, batch, static_cast<const C*>(init), init_rho ? plan->state_elems : dim,
       init_batched & 1, dm && init && !init_rho ? 1 : 0);
   JQ_CUDA(cudaGetLastError());
+  if (frame) {
+    if ((rc = frame_forward(plan, T->frame, S, batch, bmat, sm_count(), st))) return rc;
+    return measure<R>(plan, T, batch, out_type, S, out, st, true);
+  }
   if ((rc = run_passes<R>(plan, plan->fwd, T->fwd_ops, T->fwd_steps, T->fwd_rops, T, S, batch, bmat, 0, plan->fwd.passes.size(), st,
                           static_cast<const JitModule*>(T->jit)))) return rc;
   return measure<R>(plan, T, batch, out_type, S, out, st);
@@ -2488,7 +2502,8 @@ int sweep_impl(const jq_plan* plan, int batch, const double* angles, const void*
                size_t ws_bytes, cudaStream_t st) {
   using C = typename CplxT<R>::T;
   const DeviceTables* T = nullptr;
-  int rc = device_tables(plan, &T);
+  const bool frame = plan->frame.on;  // such a plan's buffers are its own
+  int rc = device_tables(plan, &T, !frame, st);
   if (rc) return rc;
   if ((rc = set_smem_attrs<R>())) return rc;
   WsLayout L = layout(plan, batch, 0);
@@ -2499,21 +2514,23 @@ int sweep_impl(const jq_plan* plan, int batch, const double* angles, const void*
   char* w = static_cast<char*>(ws);
   C* bmat = reinterpret_cast<C*>(w + L.bmat);
   double2* scratch = reinterpret_cast<double2*>(w + L.scratch);
-  if ((rc = prep<R>(plan, T, batch, angles, mats, bmat, scratch, st))) return rc;
+  if ((rc = prep<R>(plan, T, batch, angles, mats, bmat, scratch, st, frame))) return rc;
+  if (frame) return frame_forward(plan, T->frame, state, batch, bmat, sm_count(), st);
   return run_passes<R>(plan, plan->fwd, T->fwd_ops, T->fwd_steps, T->fwd_rops, T, static_cast<C*>(state), batch, bmat, 0,
                        plan->fwd.passes.size(), st, static_cast<const JitModule*>(T->jit));
 }
 
 template <typename R>
 int seed_sv(const jq_plan* plan, const DeviceTables* T, int batch, int out_type, const typename CplxT<R>::T* psi,
-            const double* ct, const void* ct_state, typename CplxT<R>::T* lam, cudaStream_t st) {
+            const double* ct, const void* ct_state, typename CplxT<R>::T* lam, cudaStream_t st,
+            bool frame = false) {
   using C = typename CplxT<R>::T;
   const int64_t dim = 1LL << plan->n_qubits;
   const int threads = 256;
   switch (out_type) {
     case JQ_OUT_EXPVAL: {
-      const std::vector<DevObs>& pobs = plan->frame.on ? plan->frame_obs : plan->obs;
-      const DevObs* od = static_cast<const DevObs*>(plan->frame.on ? T->frame_obs : T->obs_desc);
+      const std::vector<DevObs>& pobs = frame ? plan->frame_obs : plan->obs;
+      const DevObs* od = static_cast<const DevObs*>(frame ? T->frame_obs : T->obs_desc);
       const int n = plan->n_qubits, n_obs = static_cast<int>(pobs.size());
       bool zstr = n >= 9;
       for (const DevObs& o : pobs) zstr = zstr && o.kind == JQ_OBS_PAULI && o.x_mask == 0 && o.n_y == 0;
@@ -2609,7 +2626,8 @@ int adjoint_impl(const jq_plan* plan, int batch, const double* angles, const voi
     return JQ_EINVAL;
   }
   const DeviceTables* T = nullptr;
-  int rc = device_tables(plan, &T);
+  const bool frame = frame_call(plan, out_type);
+  int rc = device_tables(plan, &T, !frame, st);
   if (rc) return rc;
   if ((rc = set_smem_attrs<R>())) return rc;
   WsLayout L = layout(plan, batch, 1);
@@ -2624,12 +2642,12 @@ int adjoint_impl(const jq_plan* plan, int batch, const double* angles, const voi
   C* psi = reinterpret_cast<C*>(w + L.psi);
   double2* gacc = reinterpret_cast<double2*>(w + L.gacc);
   const int64_t elems = plan->state_elems;
-  if ((rc = prep<R>(plan, T, batch, angles, mats, bmat, scratch, st))) return rc;
+  if ((rc = prep<R>(plan, T, batch, angles, mats, bmat, scratch, st, frame))) return rc;
   const bool want_grad = (grad_angles || grad_mats) && plan->grad_stride > 0;
   if (want_grad) JQ_CUDA(cudaMemsetAsync(gacc, 0, 16 * static_cast<size_t>(plan->grad_stride) * batch, st));
-  if (plan->frame.on) {
+  if (frame) {
     // the first pass reads `state` and writes psi, so no copy precedes it
-    if ((rc = seed_sv<R>(plan, T, batch, out_type, static_cast<const C*>(state), ct, ct_state, lam, st))) return rc;
+    if ((rc = seed_sv<R>(plan, T, batch, out_type, static_cast<const C*>(state), ct, ct_state, lam, st, true))) return rc;
     const int64_t gs = 2 * plan->grad_stride;
     double* ga = reinterpret_cast<double*>(gacc);
     if ((rc = frame_adjoint(plan, T->frame, state, psi, lam, batch, bmat, want_grad ? ga : nullptr, gs, sm_count(), st)))
@@ -2688,7 +2706,7 @@ int backward_impl(const jq_plan* plan, int batch, const double* angles, const vo
   using C = typename CplxT<R>::T;
   const DeviceTables* T = nullptr;
   const bool pauli = pauli_call(plan, out_type, init) && !grad_init;
-  int rc = device_tables(plan, &T, !pauli);
+  int rc = device_tables(plan, &T, !pauli, st);
   if (rc) return rc;
   if ((rc = set_smem_attrs<R>())) return rc;
   WsLayout L = layout(plan, batch, 2);
@@ -3166,8 +3184,11 @@ int jq_forward_noalloc(const jq_plan* plan, int batch, const double* angles, con
       g_noalloc_ptr.emplace_back(dev, ws);
     }
   }
-  return jq_forward(plan, batch, angles, mats, init, init_batched, out_type, state, out, ws, JQ_STATIC_WS_BYTES,
+  tl_no_build = true;
+  rc = jq_forward(plan, batch, angles, mats, init, init_batched, out_type, state, out, ws, JQ_STATIC_WS_BYTES,
                     stream);
+  tl_no_build = false;
+  return rc;
 }
 
 // ---------------------------------------------------------------------------

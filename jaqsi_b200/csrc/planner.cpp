@@ -934,7 +934,7 @@ int build_plan(const jq_op* ops, int n_ops, const jq_obs* obs, int n_obs, int n_
   }
   // ---- frame plan (frame.h): expectation values of Z strings on a statevector of
   // one-wire unitaries and affine permutations, default tuning -----------------
-  if (!zt.empty() && tune->jit == 0 && tune->tile_bits == 0 && tune->tile_bits_adj == 0 && tune->threads == 0 &&
+  if (!zt.empty() && tune->expval_only > 1 && tune->jit == 0 && tune->tile_bits == 0 && tune->tile_bits_adj == 0 && tune->threads == 0 &&
       !no_fuse && nb >= 9) {
     std::vector<FrameOp> fops;
     bool ok = true;
@@ -980,7 +980,7 @@ int build_plan(const jq_op* ops, int n_ops, const jq_obs* obs, int n_obs, int n_
   // ---- Pauli-basis plan (pauli.cu): Pauli expectation values of a density matrix
   // under one-qubit gates, one-qubit trace-preserving channels and linear basis
   // permutations, default tuning, 5 qubits or more (tiles of 10 or 11 bits) ------
-  if (tune && tune->expval_only && mode == JQ_DENSITY && n_obs > 0 && tune->jit == 0 && tune->tile_bits == 0 &&
+  if (tune && tune->expval_only > 1 && mode == JQ_DENSITY && n_obs > 0 && tune->jit == 0 && tune->tile_bits == 0 &&
       tune->tile_bits_adj == 0 && tune->threads == 0 && tune->ckpt_stride == 0 && !no_fuse && n >= 5) {
     bool ok = true;
     for (int i = 0; i < n_obs; ++i) ok = ok && obs[i].kind == JQ_OBS_PAULI;

@@ -425,7 +425,7 @@ def get_plan(lw: Lowered, obs_specs, obs_key, n_qubits: int, mode: int, dtype: t
     simulation.py:777-801), a density matrix may be held as Pauli
     coefficients."""
     if obs_specs and not (tune or {}).get("no_fuse"):
-        tune = dict(tune or {}, expval_only=1)
+        tune = dict(tune or {}, expval_only=2)
     key = (lw.key, obs_key, n_qubits, mode, dtype, tuple(sorted((tune or {}).items())))
     with _PLAN_LOCK:
         plan = _PLAN_CACHE.get(key)

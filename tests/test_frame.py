@@ -298,3 +298,42 @@ def test_seed_of_many_z_strings(n, frame, dtype):
         got = np.concatenate([got[-1:], got[:-1]])
     np.testing.assert_allclose(got[: len(ref)], ref, atol=TOL[dtype] * np.abs(ct[0]).sum(), rtol=0)
     assert not params.grad[1].any()
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("n", [9, 13])
+def test_other_calls_of_a_frame_plan_run_the_circuit(n, dtype):
+    """A plan that absorbed nothing also answers for states and probabilities and
+    takes jq_backward: these run the circuit itself.  With expval_only = 1 the
+    state buffer of an expectation value is the final state."""
+    body = _circuit(n, 3 * n, 50)
+    base = np.random.default_rng(n).uniform(0, 2 * np.pi, 153)
+    obs = [jq.PauliZ(w) for w in range(n)]
+    script = jq.Script(lambda p: body(p) and None, n_qubits=n)
+    recs = to_records(script.record(torch.tensor(base)))
+    lw = sim.lower_tape(script.record(torch.tensor(base)), n)
+    specs, okey = sim._lower_obs(obs, n)
+    angles = torch.tensor([float(a) for a in lw.angles], dtype=torch.float64, device="cuda")
+    statics = [st[:10] + (1,) + st[11:] if st[3] >= 0 else st for st in lw.statics]  # every angle trainable
+    psi = O.simulate_pure(recs, n)
+    ev_ref, g_ref = O.adjoint_grad(recs, n, obs_records(obs), ct=np.ones(n))
+
+    def call(plan, out_type):
+        state, out = sim._forward_launch(plan, out_type, 1, 0, angles, None, None)
+        return state[0].cpu().numpy(), None if out is None else out[0].cpu().numpy()
+
+    plain = sim.Plan(statics, specs, n, L.JQ_STATEVECTOR, dtype, {"expval_only": 1})
+    state, ev = call(plain, L.JQ_OUT_EXPVAL)
+    np.testing.assert_allclose(state, psi, atol=TOL[dtype], rtol=0)
+    np.testing.assert_allclose(ev, ev_ref, atol=TOL[dtype], rtol=0)
+    plan = sim.Plan(statics, specs, n, L.JQ_STATEVECTOR, dtype, {"expval_only": 2})
+    np.testing.assert_allclose(call(plan, L.JQ_OUT_EXPVAL)[1], ev_ref, atol=TOL[dtype], rtol=0)
+    np.testing.assert_allclose(call(plan, L.JQ_OUT_STATE)[0], psi, atol=TOL[dtype], rtol=0)
+    np.testing.assert_allclose(call(plan, L.JQ_OUT_PROBS)[1], np.abs(psi) ** 2, atol=TOL[dtype], rtol=0)
+    grad = torch.empty((1, len(lw.angles)), dtype=torch.float64, device="cuda")
+    ct = torch.ones((1, n), dtype=torch.float64, device="cuda")
+    wsb = plan.workspace_bytes(1, 2)
+    ws = torch.empty(wsb, dtype=torch.uint8, device="cuda")
+    L.check(plan._lib.jq_backward(plan.handle, 1, sim._ptr(angles), None, None, 0, L.JQ_OUT_EXPVAL, sim._ptr(ct), None,
+                                  sim._ptr(grad), None, None, sim._ptr(ws), wsb, sim._stream()))
+    np.testing.assert_allclose(grad[0].cpu().numpy(), g_ref, atol=TOL[dtype] * n, rtol=0)
