@@ -54,11 +54,11 @@ sys.path.insert(0, ROOT)
 
 METRIC = "adjoint grads/sec (batched) vs plain GPU sim at ≤1e-5 err; gate-pass HBM GB/s"
 N_QUBITS, LAYERS, SEED = 24, 20, 2
-# DRAM bytes per launch of the specialised tile pass, from one ncu capture
-# (--set full, 2 launches of the 24-qubit complex64 sweep): reads 134.25 MB
-# (the whole state once) + writes 74.5 / 75.6 MB (the rest of the write-back
-# is still in the 126 MB L2 when the launch ends).
-TILE_PASS_TRAFFIC = {(24, "c64"): 209.3e6}
+# DRAM bytes per launch of the frame pass, from one ncu capture (2 launches of
+# the 24-qubit complex64 sweep): reads 134.27 MB (the whole state once) + writes
+# 74.8 / 74.9 MB (the rest of the write-back is still in the 126 MB L2 when the
+# launch ends).
+TILE_PASS_TRAFFIC = {(24, "c64"): 209.1e6}
 # Shared-memory bandwidth of one B200, nominal: 148 SMs x 128 B/clock x 1.965 GHz.
 SMEM_NOMINAL_GBS = 148 * 128 * 1.965
 
@@ -809,17 +809,17 @@ def noisy_dm_leg(dev, sets, steps, cpu, hbm_peak, world=1, max_over_ranks=None, 
         elem = 8 if name == "c64" else 16
         S = 4 ** n
         P = plan.info["n_passes_fwd"]
-        s = math.ceil(math.sqrt(P))
-        # forward, checkpoint writes, one recompute of the forward, and a reverse
-        # pass reading rho and lambda and writing lambda per forward pass
-        bytes_ = (2 * P + 1 + math.ceil(P / s) + 2 * P + 3 * P) * S * elem
+        # real Pauli coefficients, half an element each: the forward, the reverse
+        # call's own forward, and a reverse pass reading values and lambda and
+        # writing lambda per forward pass (segments run once more are not counted)
+        bytes_ = (2 * P + 2 * P + 3 * P) * S * elem // 2
         achieved = bytes_ / (dev_ms * 1e-3) / 1e9
         out[name] = {
             "ms_per_grad": ms / sets, "s_per_step": ms * 1e-3, "device_ms_per_grad": dev_ms, "passes_fwd": P,
             "algorithmic_bytes_per_grad": bytes_,
             "roofline": {"achieved": achieved, "unit": "GB/s", "frac": achieved / hbm_peak,
-                         "bytes_def": "2P (forward) + P/ceil(sqrt P) checkpoints + 2P (recompute) + 3P (reverse) "
-                                      "state transfers"},
+                         "bytes_def": "2P (forward) + 2P (forward of the reverse call) + 3P (reverse) transfers of "
+                                      "4^n real Pauli coefficients"},
             "max_abs_grad_err_vs_central_fd": float(np.abs(g0[idx] - fd).max()),
         }
         del d
@@ -883,7 +883,7 @@ def ours_arm(args):
     ref_bytes = (2 * p_ref + N_QUBITS - 1) * S * elem
     peak, peak_kind = _peaks()
     achieved = P * sw["pass_bytes"] / (sw["sweep_ms"] * 1e-3) / 1e9
-    launches = (2 + P + sw["meas_reads"]) * args.steps
+    launches = (1 + P + sw["meas_reads"]) * args.steps
     result = {
         "metric": METRIC, "value": value, "unit": "GB/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": sw["step_ms"], "higher_is_better": True, "scaling": "weak",
@@ -892,9 +892,9 @@ def ours_arm(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": TILE_PASS_TRAFFIC.get((N_QUBITS, args.dtype)),
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per launch of the "
-                                       "specialised tile pass (2 launches captured, averaged)",
+                                       "frame pass (2 launches captured, averaged)",
                      "peak_kind": peak_kind,
-                     "kernel": "jqk* (tile pass specialised per plan by NVRTC)",
+                     "kernel": "k_frame_fwd (tile pass in a moving frame)",
                      "launches_per_step": P,
                      "avg_launch_us": sw["sweep_ms"] * 1e3 / P, "bytes_per_launch": sw["pass_bytes"]},
         "e2e": {"value": e2e_value, "unit": "GB/s", "ms_per_step": sw["e2e_ms"],

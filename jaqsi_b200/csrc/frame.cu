@@ -183,7 +183,7 @@ __device__ __forceinline__ void pass_tables(const FrameStage* __restrict__ st, i
 template <typename C, int T, int MINB>
 __global__ void __launch_bounds__(1 << (T - 4), MINB)
     k_frame_fwd(C* __restrict__ state, const PassArg P, const FrameStage* __restrict__ stages,
-                const C* __restrict__ bmat, int64_t bstride, int batch, int rev) {
+                const C* __restrict__ bmat, int64_t bstride, int batch, int rev, int zero) {
   constexpr int LT = T - 4, NT = 1 << LT;
   constexpr uint32_t TB = sizeof(C) << T;     // bytes of a tile
   const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
@@ -208,6 +208,14 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
   const uint64_t rmask = rev ? tiles_per - 1 : 0;
   auto load = [&](uint32_t dst, int64_t tl) {
     const uint32_t rep = tile_rep((static_cast<uint64_t>(tl) & (tiles_per - 1)) ^ rmask, opos_lane, P.nouter);
+    if (zero) {  // the first pass of a run from |0..0>: nothing to read (24 qubits 3.09 -> 3.06 ms)
+      copy.each(P, rep, dst, [&](uint32_t a, uint32_t b) {
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (a == 0) (sizeof(C) == 8 ? v.x : v.y) = sizeof(C) == 8 ? 0x3f800000u : 0x3ff00000u;  // 1
+        *reinterpret_cast<uint4*>(smem + b) = v;
+      });
+      return;
+    }
     const C* src = state + ((tl >> P.nouter) << P.nb);
     copy.each(P, rep, dst, [&](uint32_t a, uint32_t b) { cp_async16(sbase + b, src + a); });
   };
@@ -215,7 +223,7 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
   // written; a later one starts after the first has begun.  So the tables of the
   // first tile need no wait, only the states do: 20 qubits, forward + adjoint, 108
   // passes each way: 3.26 -> 3.09 ms with the adjoint passes launched ahead as
-  // well, 2.70 ms with the tables formed before the wait; 24 qubits, 53 forward
+  // well, 2.70 ms with the tables formed before the wait; 24 qubits, 40 forward
   // passes: 3.20 -> 3.09 ms.
   int64_t last = -1;
   if (blockIdx.x < ntiles) {
@@ -491,11 +499,15 @@ template <typename C>
 __global__ void __launch_bounds__(kPrepThreads)
     k_frame_prep(const FrameGate* __restrict__ gates, int ngates, const DevBlock* __restrict__ blocks,
                  const DevPrim* __restrict__ prims, const DevOp* __restrict__ ops, const double* __restrict__ angles,
-                 int n_angles, const double2* __restrict__ cpool, C* __restrict__ bmat, int64_t bstride) {
+                 int n_angles, const double2* __restrict__ cpool, C* __restrict__ bmat, int64_t bstride, ZeroFill z) {
   __shared__ uint32_t wsum[kPrepThreads / 32];
   const int64_t inst = blockIdx.x;
   const double* ang = angles ? angles + inst * n_angles : nullptr;
   C* bm = bmat + inst * bstride;
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    for (int64_t i = inst * kPrepThreads + threadIdx.x; i < z.n[k]; i += static_cast<int64_t>(gridDim.x) * kPrepThreads)
+      z.p[k][i] = 0.0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t carry = 0;
   for (int g0 = 0; g0 < ngates; g0 += kPrepThreads) {
@@ -656,7 +668,8 @@ template <typename C> int upload_shapes(const FramePlan& fp, FrameDev* d) {
 }
 
 template <typename C>
-int forward_t(const jq_plan* plan, const FrameDev& d, C* state, int batch, const C* bmat, int sm_count, cudaStream_t st) {
+int forward_t(const jq_plan* plan, const FrameDev& d, C* state, int batch, const C* bmat, bool from_zero, int sm_count,
+              cudaStream_t st) {
   const FramePlan& fp = plan->frame;
   const bool pdl = pdl_on(st);
   for (size_t i = 0; i < fp.passes.size(); ++i) {
@@ -675,8 +688,8 @@ int forward_t(const jq_plan* plan, const FrameDev& d, C* state, int batch, const
     cfg.numAttrs = pdl && i > 0 ? 1 : 0;
     const FrameStage* sp = d.stages;
     int64_t bs = plan->bmat_stride;
-    int rev = static_cast<int>(i & 1);
-    void* args[] = {&state, &a, &sp, &bmat, &bs, &batch, &rev};
+    int rev = static_cast<int>(i & 1), zero = from_zero && i == 0;
+    void* args[] = {&state, &a, &sp, &bmat, &bs, &batch, &rev, &zero};
     JQ_CUDA(cudaLaunchKernelExC(&cfg, fwd_kernel<C>(p), args));
   }
   return JQ_OK;
@@ -739,25 +752,27 @@ void frame_free(FrameDev* d) {
 }
 
 int frame_prep(const jq_plan* plan, const FrameDev& d, const DevBlock* blocks, const DevPrim* prims, const DevOp* ops,
-               const double* cpool, int batch, const double* angles, void* bmat, cudaStream_t st) {
+               const double* cpool, int batch, const double* angles, void* bmat, const ZeroFill& z, cudaStream_t st) {
   const int ng = static_cast<int>(plan->frame.gates.size());
-  if (ng == 0) return JQ_OK;
+  if (ng == 0 && z.n[0] + z.n[1] == 0) return JQ_OK;
   const double2* cp = reinterpret_cast<const double2*>(cpool);
   if (plan->dtype == JQ_C64)
     k_frame_prep<float2><<<batch, kPrepThreads, 0, st>>>(d.gates, ng, blocks, prims, ops, angles, plan->n_angles, cp,
-                                                         static_cast<float2*>(bmat), plan->bmat_stride);
+                                                         static_cast<float2*>(bmat), plan->bmat_stride, z);
   else
     k_frame_prep<double2><<<batch, kPrepThreads, 0, st>>>(d.gates, ng, blocks, prims, ops, angles, plan->n_angles, cp,
-                                                          static_cast<double2*>(bmat), plan->bmat_stride);
+                                                          static_cast<double2*>(bmat), plan->bmat_stride, z);
   JQ_CUDA(cudaGetLastError());
   return JQ_OK;
 }
 
-int frame_forward(const jq_plan* plan, const FrameDev& d, void* state, int batch, const void* bmat, int sm_count,
-                  cudaStream_t st) {
+int frame_forward(const jq_plan* plan, const FrameDev& d, void* state, int batch, const void* bmat, bool from_zero,
+                  int sm_count, cudaStream_t st) {
   return plan->dtype == JQ_C64
-             ? forward_t<float2>(plan, d, static_cast<float2*>(state), batch, static_cast<const float2*>(bmat), sm_count, st)
-             : forward_t<double2>(plan, d, static_cast<double2*>(state), batch, static_cast<const double2*>(bmat), sm_count, st);
+             ? forward_t<float2>(plan, d, static_cast<float2*>(state), batch, static_cast<const float2*>(bmat), from_zero,
+                                 sm_count, st)
+             : forward_t<double2>(plan, d, static_cast<double2*>(state), batch, static_cast<const double2*>(bmat), from_zero,
+                                  sm_count, st);
 }
 
 int frame_adjoint(const jq_plan* plan, const FrameDev& d, const void* psi_in, void* psi, void* lam, int batch,

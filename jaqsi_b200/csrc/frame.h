@@ -110,10 +110,16 @@ bool frame_schedule(const std::vector<FrameOp>& ops, int nb, int t_max, int c, i
 int frame_upload(const jq_plan* plan, FrameDev* d);
 int frame_tables(const FramePlan& fp, FrameDev* d);  // the tables alone
 void frame_free(FrameDev* d);
+// Arrays the gate matrices' kernel sets to zero for the kernels after it.
+struct ZeroFill {
+  double* p[2] = {nullptr, nullptr};
+  int64_t n[2] = {0, 0};
+};
 int frame_prep(const jq_plan* plan, const FrameDev& d, const DevBlock* blocks, const DevPrim* prims, const DevOp* ops,
-               const double* cpool, int batch, const double* angles, void* bmat, cudaStream_t st);
-int frame_forward(const jq_plan* plan, const FrameDev& d, void* state, int batch, const void* bmat, int sm_count,
-                  cudaStream_t st);
+               const double* cpool, int batch, const double* angles, void* bmat, const ZeroFill& z, cudaStream_t st);
+// from_zero: the states start at |0..0> and hold nothing yet (a plan with passes)
+int frame_forward(const jq_plan* plan, const FrameDev& d, void* state, int batch, const void* bmat, bool from_zero,
+                  int sm_count, cudaStream_t st);
 // psi_in: final state (read by the first launched pass only), psi: workspace
 // for the rest; gacc: 3 doubles a gate with cotangents, instance stride gstride doubles.
 int frame_adjoint(const jq_plan* plan, const FrameDev& d, const void* psi_in, void* psi, void* lam, int batch,

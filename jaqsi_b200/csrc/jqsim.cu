@@ -2356,11 +2356,9 @@ int run_passes(const jq_plan* plan, const Schedule& sch, const TileOp* dops, con
 
 template <typename R>
 int prep(const jq_plan* plan, const DeviceTables* T, int batch, const double* angles, const void* mats,
-         typename CplxT<R>::T* bmat, double2* scratch, cudaStream_t st, bool frame = false) {
+         typename CplxT<R>::T* bmat, double2* scratch, cudaStream_t st) {
   const int nbk = static_cast<int>(plan->blocks.size());
   if (nbk == 0) return JQ_OK;
-  if (frame)
-    return frame_prep(plan, T->frame, T->blocks, T->prims, T->ops, T->const_pool, batch, angles, bmat, st);
   const int64_t work = static_cast<int64_t>(nbk) * batch;
   const int threads = 128;
   const int grid = static_cast<int>((work + threads - 1) / threads);
@@ -2374,7 +2372,7 @@ int prep(const jq_plan* plan, const DeviceTables* T, int batch, const double* an
 
 template <typename R>
 int measure(const jq_plan* plan, const DeviceTables* T, int batch, int out_type, const typename CplxT<R>::T* state,
-            void* out, cudaStream_t st, bool frame = false) {
+            void* out, cudaStream_t st, bool frame = false /* its values are zero already */) {
   using C = typename CplxT<R>::T;
   const int n = plan->n_qubits;
   const int64_t dim = 1LL << n;
@@ -2394,7 +2392,7 @@ int measure(const jq_plan* plan, const DeviceTables* T, int batch, int out_type,
     const int n_obs = static_cast<int>(plan->obs.size());
     if (n_obs == 0) return JQ_OK;
     double* o = static_cast<double*>(out);
-    JQ_CUDA(cudaMemsetAsync(o, 0, sizeof(double) * n_obs * batch, st));
+    if (!frame) JQ_CUDA(cudaMemsetAsync(o, 0, sizeof(double) * n_obs * batch, st));
     const std::vector<DevObs>& pobs = frame ? plan->frame_obs : plan->obs;
     const DevObs* od = static_cast<const DevObs*>(frame ? T->frame_obs : T->obs_desc);
     const double2* pool = reinterpret_cast<const double2*>(T->obs_pool);
@@ -2479,17 +2477,26 @@ int forward_impl(const jq_plan* plan, int batch, const double* angles, const voi
   C* bmat = reinterpret_cast<C*>(w + L.bmat);
   if (pauli) return pauli_forward(plan, *T, batch, angles, state, bmat, static_cast<double*>(out), sm_count(), st);
   double2* scratch = reinterpret_cast<double2*>(w + L.scratch);
-  if ((rc = prep<R>(plan, T, batch, angles, mats, bmat, scratch, st, frame))) return rc;
+  if (frame) {
+    ZeroFill z;
+    z.p[0] = static_cast<double*>(out);
+    z.n[0] = out ? static_cast<int64_t>(plan->obs.size()) * batch : 0;
+    rc = frame_prep(plan, T->frame, T->blocks, T->prims, T->ops, T->const_pool, batch, angles, bmat, z, st);
+  } else {
+    rc = prep<R>(plan, T, batch, angles, mats, bmat, scratch, st);
+  }
+  if (rc) return rc;
   C* S = static_cast<C*>(state);
   const bool dm = plan->mode == JQ_DENSITY;
   const int64_t dim = 1LL << plan->n_qubits;
   const bool init_rho = dm && init && (init_batched & JQ_INIT_DENSITY);  // init is a density matrix
-  k_init<R><<<grid_for(plan->state_elems * batch, 256), 256, 0, st>>>(
+  const bool from_zero = frame && !init && !plan->frame.passes.empty();  // its first pass writes every amplitude
+  if (!from_zero) k_init<R><<<grid_for(plan->state_elems * batch, 256), 256, 0, st>>>(
       S, plan->state_elems, batch, static_cast<const C*>(init), init_rho ? plan->state_elems : dim,
       init_batched & 1, dm && init && !init_rho ? 1 : 0);
   JQ_CUDA(cudaGetLastError());
   if (frame) {
-    if ((rc = frame_forward(plan, T->frame, S, batch, bmat, sm_count(), st))) return rc;
+    if ((rc = frame_forward(plan, T->frame, S, batch, bmat, from_zero, sm_count(), st))) return rc;
     return measure<R>(plan, T, batch, out_type, S, out, st, true);
   }
   if ((rc = run_passes<R>(plan, plan->fwd, T->fwd_ops, T->fwd_steps, T->fwd_rops, T, S, batch, bmat, 0, plan->fwd.passes.size(), st,
@@ -2514,8 +2521,11 @@ int sweep_impl(const jq_plan* plan, int batch, const double* angles, const void*
   char* w = static_cast<char*>(ws);
   C* bmat = reinterpret_cast<C*>(w + L.bmat);
   double2* scratch = reinterpret_cast<double2*>(w + L.scratch);
-  if ((rc = prep<R>(plan, T, batch, angles, mats, bmat, scratch, st, frame))) return rc;
-  if (frame) return frame_forward(plan, T->frame, state, batch, bmat, sm_count(), st);
+  if (frame) {
+    rc = frame_prep(plan, T->frame, T->blocks, T->prims, T->ops, T->const_pool, batch, angles, bmat, ZeroFill(), st);
+    return rc ? rc : frame_forward(plan, T->frame, state, batch, bmat, false, sm_count(), st);
+  }
+  if ((rc = prep<R>(plan, T, batch, angles, mats, bmat, scratch, st))) return rc;
   return run_passes<R>(plan, plan->fwd, T->fwd_ops, T->fwd_steps, T->fwd_rops, T, static_cast<C*>(state), batch, bmat, 0,
                        plan->fwd.passes.size(), st, static_cast<const JitModule*>(T->jit));
 }
@@ -2642,25 +2652,29 @@ int adjoint_impl(const jq_plan* plan, int batch, const double* angles, const voi
   C* psi = reinterpret_cast<C*>(w + L.psi);
   double2* gacc = reinterpret_cast<double2*>(w + L.gacc);
   const int64_t elems = plan->state_elems;
-  if ((rc = prep<R>(plan, T, batch, angles, mats, bmat, scratch, st, frame))) return rc;
   const bool want_grad = (grad_angles || grad_mats) && plan->grad_stride > 0;
-  if (want_grad) JQ_CUDA(cudaMemsetAsync(gacc, 0, 16 * static_cast<size_t>(plan->grad_stride) * batch, st));
   if (frame) {
     // the first pass reads `state` and writes psi, so no copy precedes it
-    if ((rc = seed_sv<R>(plan, T, batch, out_type, static_cast<const C*>(state), ct, ct_state, lam, st, true))) return rc;
     const int64_t gs = 2 * plan->grad_stride;
     double* ga = reinterpret_cast<double*>(gacc);
+    ZeroFill z;
+    z.p[0] = ga;
+    z.n[0] = want_grad ? gs * batch : 0;
+    z.p[1] = grad_angles;
+    z.n[1] = grad_angles ? static_cast<int64_t>(plan->n_angles) * batch : 0;
+    if ((rc = frame_prep(plan, T->frame, T->blocks, T->prims, T->ops, T->const_pool, batch, angles, bmat, z, st))) return rc;
+    if ((rc = seed_sv<R>(plan, T, batch, out_type, static_cast<const C*>(state), ct, ct_state, lam, st, true))) return rc;
     if ((rc = frame_adjoint(plan, T->frame, state, psi, lam, batch, bmat, want_grad ? ga : nullptr, gs, sm_count(), st)))
       return rc;
     if (grad_init) JQ_CUDA(cudaMemcpyAsync(grad_init, lam, sizeof(C) * elems * batch, cudaMemcpyDeviceToDevice, st));
-    if (grad_angles && plan->n_angles > 0)
-      JQ_CUDA(cudaMemsetAsync(grad_angles, 0, sizeof(double) * plan->n_angles * batch, st));
     if (grad_mats && plan->n_mats > 0)
       JQ_CUDA(cudaMemsetAsync(grad_mats, 0, 16 * static_cast<size_t>(plan->n_mats) * batch, st));
     if (!want_grad) return JQ_OK;
     return frame_chain(plan, T->frame, T->blocks, T->prims, T->ops, T->const_pool, batch, angles, bmat, ga, gs,
                        grad_angles, st);
   }
+  if ((rc = prep<R>(plan, T, batch, angles, mats, bmat, scratch, st))) return rc;
+  if (want_grad) JQ_CUDA(cudaMemsetAsync(gacc, 0, 16 * static_cast<size_t>(plan->grad_stride) * batch, st));
   JQ_CUDA(cudaMemcpyAsync(psi, state, sizeof(C) * elems * batch, cudaMemcpyDeviceToDevice, st));
   if ((rc = seed_sv<R>(plan, T, batch, out_type, psi, ct, ct_state, lam, st))) return rc;
   // Specialised adjoint: the forward schedule's passes in reverse, each one
@@ -2990,6 +3004,14 @@ int jq_plan_get_info(const jq_plan* plan, jq_plan_info* info) {
   }
   if (plan->frame.on) {
     const FramePlan& f = plan->frame;
+    info->n_passes_fwd = info->n_passes_adj = static_cast<int32_t>(f.passes.size());
+    info->n_tile_ops_fwd = static_cast<int32_t>(f.gates.size());
+    info->n_stages_fwd = static_cast<int32_t>(f.stages.size());
+    info->n_smem_ops_fwd = 0;
+    if (!f.passes.empty()) info->tile_bits_fwd = info->tile_bits_adj = f.passes[0].t;
+  }
+  if (plan->pauli.on) {
+    const FramePlan& f = plan->pauli;
     info->n_passes_fwd = info->n_passes_adj = static_cast<int32_t>(f.passes.size());
     info->n_tile_ops_fwd = static_cast<int32_t>(f.gates.size());
     info->n_stages_fwd = static_cast<int32_t>(f.stages.size());

@@ -337,3 +337,31 @@ def test_other_calls_of_a_frame_plan_run_the_circuit(n, dtype):
     L.check(plan._lib.jq_backward(plan.handle, 1, sim._ptr(angles), None, None, 0, L.JQ_OUT_EXPVAL, sim._ptr(ct), None,
                                   sim._ptr(grad), None, None, sim._ptr(ws), wsb, sim._stream()))
     np.testing.assert_allclose(grad[0].cpu().numpy(), g_ref, atol=TOL[dtype] * n, rtol=0)
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("n", [9, 12, 13])
+@pytest.mark.parametrize("gates", [0, 1])
+def test_frame_runs_that_start_at_zero(n, gates, dtype):
+    """The first pass writes the start state: of no gate (no pass), of one, and
+    over memory that holds something else."""
+    torch.full((1 << 22,), float("nan"), device="cuda")  # freed at once: the call's buffers land on it
+
+    def body(p):
+        jq.PauliX(wires=n - 1)
+        jq.CX(wires=[n - 1, 0])
+        if gates:
+            jq.RX(p[0], wires=0)
+            jq.CX(wires=[0, 3])
+
+    base = np.array([0.7])
+    obs = [jq.PauliZ(w) for w in range(n)]
+    script = jq.Script(lambda p: body(p) and None, n_qubits=n)
+    params = torch.tensor(base, requires_grad=True)
+    ev = script.execute("expval", obs, args=(params,), dtype=dtype)
+    want = O.expval_state(O.simulate_pure(to_records(script.record(torch.tensor(base))), n), n, obs_records(obs))
+    np.testing.assert_allclose(ev.detach().cpu().numpy(), want, atol=TOL[dtype], rtol=0)
+    if gates:
+        ev.sum().backward()
+        _, g = O.adjoint_grad(to_records(script.record(torch.tensor(base))), n, obs_records(obs), ct=np.ones(n))
+        np.testing.assert_allclose(params.grad.numpy(), g, atol=TOL[dtype] * n, rtol=0)
