@@ -175,9 +175,9 @@ __device__ __forceinline__ void pass_tables(const FrameStage* __restrict__ st, i
 //
 // Bound by instruction issue and its latencies (58% of issue slots, 120
 // instructions an amplitude and pass of 14 gates, 65 of them FP32; shared memory
-// 51%, HBM 40% busy).  24 qubits, 20 layers, complex64: 40 passes of 80 us for 133
-// stages against 66 passes of 60 us for 157, 4.20 -> 3.28 ms a call (3.55 with
-// tiles copied 8 bytes at a time instead of 16).  Five CTAs an SM; six (79
+// 51%, HBM 40% busy).  24 qubits, 20 layers, complex64: 40 passes of 75 us for 133
+// stages against 66 passes of 60 us for 157, 4.19 -> 3.06 ms a call (tiles copied 8
+// bytes at a time instead of 16 cost 0.27 ms).  Five CTAs an SM; six (79
 // registers) were 18% slower.  Pairs of amplitudes in packed FMAs
 // throughout: 1.5 times slower, register moves for every packed operand.
 template <typename C, int T, int MINB>
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
 // other gates of its stage, and the generators of a rotation see only these
 // three of its eight numbers.  Partial sums in the run precision per tile and
 // warp, float64 across tiles.  20 qubits, 50 layers, complex64 (forward +
-// adjoint): 4.76 -> 2.67 ms a call; 16 qubits, 9 layers, complex128, three sets:
+// adjoint): 4.76 -> 2.60 ms a call; 16 qubits, 9 layers, complex128, three sets:
 // 0.93 -> 0.43 ms.
 template <typename C, int T, int MINB>
 __global__ void __launch_bounds__(1 << (T - 4), MINB)

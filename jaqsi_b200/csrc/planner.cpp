@@ -963,7 +963,8 @@ int build_plan(const jq_op* ops, int n_ops, const jq_obs* obs, int n_obs, int n_
     }
     // States of up to 12 bits are one tile.  Larger ones take tiles of 11 bits:
     // at 24 qubits complex64 10, 11 and 12 bits measured 3.62, 3.63 and 3.81 ms,
-    // at 20 qubits (forward + adjoint) 3.98, 3.63 and 3.62 ms.  Runs of 64 bytes
+    // at 20 qubits (forward + adjoint) 3.98, 3.63 and 3.62 ms; with passes launched
+    // ahead 3.17, 3.10, 3.29 and 2.89, 2.69, 2.81 ms.  Runs of 64 bytes
     // (3 low bits) leave more of a tile to the masks; beyond the L2 (126 MB) runs of
     // 128 bytes are faster in spite of more passes: 24 qubits 3.51 against 3.63 ms,
     // 20 qubits 3.87 against 3.63 ms.
