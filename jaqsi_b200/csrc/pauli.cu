@@ -220,7 +220,8 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
     const F* src = in + ((tl >> P.nouter) << P.nb);
     copy.each(P, rep_of(tl), dst, [&](uint32_t a, uint32_t b) { cp_async16(sbase + b, src + a); });
   };
-  // k_pauli_init has run since prep: the matrices need no wait, the states do
+  // the first pass of a call follows prep in plain stream order: the matrices need
+  // no wait, the states do
   int64_t last = -1;
   if (blockIdx.x < ntiles) {
     last = static_cast<int64_t>(blockIdx.x) >> P.nouter;
@@ -479,7 +480,7 @@ template <typename F>
 __global__ void k_pauli_prep(const FrameGate* __restrict__ gates, int ngates, const DevBlock* __restrict__ blocks,
                              const DevPrim* __restrict__ prims, const DevOp* __restrict__ ops,
                              const double* __restrict__ angles, int n_angles, const double2* __restrict__ cpool,
-                             F* __restrict__ bmat, int64_t bstride, int batch) {
+                             F* __restrict__ bmat, int64_t bstride, int batch, F* __restrict__ state, int nb) {
   const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= static_cast<int64_t>(batch) * ngates) return;
   const int64_t inst = idx / ngates;
@@ -494,6 +495,13 @@ __global__ void k_pauli_prep(const FrameGate* __restrict__ gates, int ngates, co
     transfer_mul(pm, acc, tmp);
     for (int i = 0; i < 12; ++i) acc[i] = tmp[i];
   }
+  // A NaN or infinite angle: not every word's value depends on this gate, but the
+  // density matrix has no finite entry left.  The coefficient of the identity, that
+  // no pass writes, tells k_pauli_expval; through the first columns of the
+  // matrices' cotangents it reaches every gradient.
+  double all = 0.0;
+  for (int i = 0; i < 12; ++i) all += acc[i];
+  if (!isfinite(all)) state[inst << nb] = static_cast<F>(all - all);
   F* o = bmat + inst * bstride + 2 * fg.mat_off;
   if (fg.diag == 1) {
     o[0] = static_cast<F>(acc[1]);
@@ -575,7 +583,8 @@ __global__ void k_pauli_expval(const F* __restrict__ s, int nb, const PauliObs* 
   if (i >= static_cast<int64_t>(n_obs) * batch) return;
   const int64_t inst = i / n_obs;
   const PauliObs o = obs[i - inst * n_obs];
-  out[i] = o.coeff * static_cast<double>(s[(inst << nb) + o.index]);
+  const F one = s[inst << nb];  // NaN: see k_pauli_prep
+  out[i] = one != one ? static_cast<double>(one) : o.coeff * static_cast<double>(s[(inst << nb) + o.index]);
 }
 template <typename F>
 __global__ void k_pauli_seed(F* __restrict__ lam, int nb, const PauliObs* __restrict__ obs, int n_obs, int batch,
@@ -650,14 +659,14 @@ unsigned blocks_for(int64_t work, int threads) { return static_cast<unsigned>((w
 template <typename F>
 int start(const jq_plan* plan, const FrameDev& d, const DeviceTables& T, int batch, const double* angles, F* bmat, F* s,
           int sms, cudaStream_t st) {
+  const int64_t total = static_cast<int64_t>(batch) << plan->n_bits;
+  k_pauli_init<F><<<std::min<unsigned>(blocks_for(total, 256), static_cast<unsigned>(sms) * 16), 256, 0, st>>>(
+      s, total, 0x55555555u & ((1u << plan->n_bits) - 1u));
   const int ng = static_cast<int>(plan->pauli.gates.size());
   if (ng > 0)
     k_pauli_prep<F><<<blocks_for(static_cast<int64_t>(ng) * batch, 64), 64, 0, st>>>(
         d.gates, ng, T.blocks, T.prims, T.ops, angles, plan->n_angles, reinterpret_cast<const double2*>(T.const_pool),
-        bmat, 2 * plan->bmat_stride, batch);
-  const int64_t total = static_cast<int64_t>(batch) << plan->n_bits;
-  k_pauli_init<F><<<std::min<unsigned>(blocks_for(total, 256), static_cast<unsigned>(sms) * 16), 256, 0, st>>>(
-      s, total, 0x55555555u & ((1u << plan->n_bits) - 1u));
+        bmat, 2 * plan->bmat_stride, batch, s, plan->n_bits);
   JQ_CUDA(cudaGetLastError());
   return JQ_OK;
 }
@@ -669,7 +678,7 @@ int forward_t(const jq_plan* plan, const FrameDev& d, const DeviceTables& T, int
   if (rc) return rc;
   const bool pdl = pdl_on(st);
   for (size_t i = 0; i < plan->pauli.passes.size(); ++i)
-    if ((rc = pass_fwd<F>(plan, d, i, s, s, batch, bmat, sms, st, pdl))) return rc;
+    if ((rc = pass_fwd<F>(plan, d, i, s, s, batch, bmat, sms, st, pdl && i > 0))) return rc;
   const int no = static_cast<int>(plan->pauli_obs.size());
   k_pauli_expval<F><<<blocks_for(static_cast<int64_t>(no) * batch, 128), 128, 0, st>>>(
       s, plan->n_bits, static_cast<const PauliObs*>(T.pauli_obs), no, batch, out);
@@ -701,7 +710,7 @@ int backward_t(const jq_plan* plan, const FrameDev& d, const DeviceTables& T, in
     for (int64_t c = 0; c + 1 < nck; ++c)  // checkpoint c + 1 from c, through the segment's buffer
       for (int64_t p = c * S; p < (c + 1) * S; ++p)
         if ((rc = pass_fwd<F>(plan, d, static_cast<size_t>(p), p == c * S ? slot(c) : seg(0),
-                              p + 1 == (c + 1) * S ? slot(c + 1) : seg(0), batch, bmat, sms, st, pdl)))
+                              p + 1 == (c + 1) * S ? slot(c + 1) : seg(0), batch, bmat, sms, st, pdl && p > 0)))
           return rc;
   JQ_CUDA(cudaMemsetAsync(lam, 0, bytes, st));
   const int no = static_cast<int>(plan->pauli_obs.size());
@@ -715,7 +724,8 @@ int backward_t(const jq_plan* plan, const FrameDev& d, const DeviceTables& T, in
     const int64_t p0 = c * S, p1 = std::min(P, p0 + S);
     auto input = [&](int64_t p) { return nck > 0 ? (p == p0 ? slot(c) : seg(p - p0 - 1)) : slot(p); };
     for (int64_t p = p0; p + 1 < p1; ++p)
-      if ((rc = pass_fwd<F>(plan, d, static_cast<size_t>(p), input(p), input(p + 1), batch, bmat, sms, st, pdl))) return rc;
+      if ((rc = pass_fwd<F>(plan, d, static_cast<size_t>(p), input(p), input(p + 1), batch, bmat, sms, st, pdl && p > 0)))
+        return rc;
     for (int64_t p = p1 - 1; p >= p0 && want; --p) {
       const FramePass& fpz = fp.passes[static_cast<size_t>(p)];
       PassArg a = pass_arg(fpz, plan->n_bits, true);
