@@ -88,72 +88,83 @@ class _ArgWatch(TorchFunctionMode):
         return out
 
 
+class _Kept:
+    """Numbers a trace keeps as a tensor on each device it is used on.  Autograd
+    saves them, on whatever stream the caller runs: they are no inference
+    tensors and belong to no torch.func level, whichever is open around the first
+    call, and their memory is not given back while another stream reads it."""
+
+    __slots__ = ("data", "dtype", "at")
+
+    def __init__(self, data, dtype):
+        self.data, self.dtype = data, dtype
+        self.at: dict = {}  # device -> (tensor, stream it was made on)
+
+    def __len__(self):
+        return len(self.data)
+
+    def on(self, device):
+        stream = torch.cuda.current_stream(device) if device.type == "cuda" else None
+        kept = self.at.get(device)
+        if kept is None:
+            with torch.inference_mode(False):
+                t = torch.tensor(self.data, dtype=self.dtype, device=device)
+                while simulation._functorch_wrapped(t):
+                    t = torch._C._functorch.get_unwrapped(t)
+            kept = self.at[device] = (t, stream)
+        t, home = kept
+        if stream != home:
+            t.record_stream(stream)
+        return t
+
+
 class _Trace:
     """Cached lowering of one call signature and where each angle comes from:
     slot positions and flat element indices per argument, plus constants."""
 
-    __slots__ = ("lw", "n_qubits", "use_density", "n_angles", "parts", "cpos", "cval", "plans", "_dev")
+    __slots__ = ("lw", "n_qubits", "use_density", "n_angles", "parts", "cpos", "cval", "plans")
 
     def __init__(self, lw, n_qubits, use_density, parts, cpos, cval):
         self.lw = lw
         self.n_qubits = n_qubits
         self.use_density = use_density
         self.n_angles = len(lw.angles)
-        self.parts = parts  # [(arg index, slot positions, flat indices)]
-        self.cpos, self.cval = cpos, cval
+        self.parts = [(i, _Kept(pos, torch.long), _Kept(idx, torch.long)) for i, pos, idx in parts]
+        self.cpos, self.cval = _Kept(cpos, torch.long), _Kept(cval, torch.float64)
         self.plans: dict = {}
-        self._dev: dict = {}
         lw.angles = []  # the first call's values are not kept
-
-    def _idx(self, dev):
-        d = self._dev.get(dev)
-        if d is None:
-            d = ([(i, torch.tensor(pos, dtype=torch.long, device=dev), {"cpu": torch.tensor(idx, dtype=torch.long)})
-                  for i, pos, idx in self.parts],
-                 torch.tensor(self.cpos, dtype=torch.long, device=dev),
-                 torch.tensor(self.cval, dtype=torch.float64, device=dev))
-            self._dev[dev] = d
-        return d
-
-    @staticmethod
-    def _on(idx, device):
-        """The element indices on an argument's device."""
-        t = idx.get(device)
-        if t is None:
-            t = idx[device] = idx["cpu"].to(device)
-        return t
 
     def angles(self, args, dev, batch=None, in_axes=None):
         """float64 angles on `dev`: [n_angles], or [batch, n_angles] with
         each argument's batch axis from in_axes (None: broadcast)."""
         if self.n_angles == 0:
             return None
-        parts, cpos, cval = self._idx(dev)
+        parts, cpos, cval = self.parts, self.cpos, self.cval
         if batch is None:
-            if len(parts) == 1 and not self.cpos and len(parts[0][2]["cpu"]) == self.n_angles and self._ordered():
+            if len(parts) == 1 and not cpos and len(parts[0][2]) == self.n_angles and self._ordered():
                 i, _, idx = parts[0]
-                return args[i].reshape(-1).index_select(0, self._on(idx, args[i].device)).to(dev, torch.float64)
+                return args[i].reshape(-1).index_select(0, idx.on(args[i].device)).to(dev, torch.float64)
             out = torch.zeros(self.n_angles, dtype=torch.float64, device=dev)
-            if self.cpos:
-                out = out.index_copy(0, cpos, cval)
+            if cpos:
+                out = out.index_copy(0, cpos.on(dev), cval.on(dev))
             for i, pos, idx in parts:
-                v = args[i].reshape(-1).index_select(0, self._on(idx, args[i].device)).to(dev, torch.float64)
-                out = out.index_copy(0, pos, v)
+                v = args[i].reshape(-1).index_select(0, idx.on(args[i].device)).to(dev, torch.float64)
+                out = out.index_copy(0, pos.on(dev), v)
             return out
         out = torch.zeros((batch, self.n_angles), dtype=torch.float64, device=dev)
-        if self.cpos:
-            out = out.index_copy(1, cpos, cval.expand(batch, -1))
+        if cpos:
+            out = out.index_copy(1, cpos.on(dev), cval.on(dev).expand(batch, -1))
         for i, pos, idx in parts:
             a, ax = args[i], in_axes[i]
             if ax is None:
-                v = a.reshape(-1).index_select(0, self._on(idx, a.device)).to(dev, torch.float64).expand(batch, -1)
+                v = a.reshape(-1).index_select(0, idx.on(a.device)).to(dev, torch.float64).expand(batch, -1)
             else:
-                v = a.movedim(ax, 0).reshape(batch, -1).index_select(1, self._on(idx, a.device)).to(dev, torch.float64)
-            out = out.index_copy(1, pos, v)
+                v = a.movedim(ax, 0).reshape(batch, -1).index_select(1, idx.on(a.device)).to(dev, torch.float64)
+            out = out.index_copy(1, pos.on(dev), v)
         return out
 
     def _ordered(self):
-        pos = self.parts[0][1]
+        pos = self.parts[0][1].data
         return all(p == k for k, p in enumerate(pos))
 
 
