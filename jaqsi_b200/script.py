@@ -98,13 +98,14 @@ class _Kept:
 
     def __init__(self, data, dtype):
         self.data, self.dtype = data, dtype
-        self.at: dict = {}  # device -> (tensor, stream it was made on)
+        self.at: dict = {}  # device -> (tensor, handle of the stream it was made on)
 
     def __len__(self):
         return len(self.data)
 
     def on(self, device):
-        stream = torch.cuda.current_stream(device) if device.type == "cuda" else None
+        # the handle alone: a Stream object takes 2 us
+        stream = torch._C._cuda_getCurrentRawStream(device.index or 0) if device.type == "cuda" else 0
         kept = self.at.get(device)
         if kept is None:
             with torch.inference_mode(False):
@@ -114,7 +115,7 @@ class _Kept:
             kept = self.at[device] = (t, stream)
         t, home = kept
         if stream != home:
-            t.record_stream(stream)
+            t.record_stream(torch.cuda.current_stream(device))
         return t
 
 
