@@ -288,11 +288,11 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
 // components Im tr(sigma_k lam psi^dagger) of each gate's cotangent, all four
 // gates of a stage at one point: a gate's reduced matrix does not depend on the
 // other gates of its stage, and the generators of a rotation see only these
-// three of its eight numbers.  Partial sums in the run precision per tile and
-// warp, float64 across tiles.  20 qubits, 50 layers, complex64 (forward +
+// three of its eight numbers.  A thread's and a warp's sums are of type A, tiles and
+// warps add up in float64.  20 qubits, 50 layers, complex64 (forward +
 // adjoint): 4.76 -> 2.60 ms a call; 16 qubits, 9 layers, complex128, three sets:
 // 0.93 -> 0.43 ms.
-template <typename C, int T, int MINB>
+template <typename C, typename A, int T, int MINB>
 __global__ void __launch_bounds__(1 << (T - 4), MINB)
     k_frame_adj(const C* psi_in, C* psi, C* __restrict__ lam, const PassArg P, const FrameStage* __restrict__ stages,
                 const C* __restrict__ bmat, int64_t bstride, double* __restrict__ gacc, int64_t gstride, int batch) {
@@ -398,26 +398,29 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
       }
       if (gacc) {
         // -<lam|sigma|psi> imaginary parts: x, y, z of gates 0..3
-        F v[16];
-        F w[16];
+        A v[16], w[16], lx[16], ly[16], px[16], py[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) w[j] = fma(l[j].y, p[j].x, -(l[j].x * p[j].y));
+        for (int j = 0; j < 16; ++j) {
+          lx[j] = l[j].x; ly[j] = l[j].y;
+          px[j] = p[j].x; py[j] = p[j].y;
+          w[j] = fma(ly[j], px[j], -(lx[j] * py[j]));
+        }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          F x0 = 0, x1 = 0, y0 = 0, y1 = 0, z = 0;
+          A x0 = 0, x1 = 0, y0 = 0, y1 = 0, z = 0;
 #pragma unroll
           for (int j = 0; j < 16; ++j)
             if (!(j >> q & 1)) {
               const int m = j | (1 << q);
               // Im(l0* p1) + Im(l1* p0), Re(l0* p1) - Re(l1* p0)
-              x0 = fma(l[j].y, p[m].x, x0);
-              x1 = fma(l[j].x, p[m].y, x1);
-              x0 = fma(l[m].y, p[j].x, x0);
-              x1 = fma(l[m].x, p[j].y, x1);
-              y0 = fma(l[j].x, p[m].x, y0);
-              y1 = fma(l[m].x, p[j].x, y1);
-              y0 = fma(l[j].y, p[m].y, y0);
-              y1 = fma(l[m].y, p[j].y, y1);
+              x0 = fma(ly[j], px[m], x0);
+              x1 = fma(lx[j], py[m], x1);
+              x0 = fma(ly[m], px[j], x0);
+              x1 = fma(lx[m], py[j], x1);
+              y0 = fma(lx[j], px[m], y0);
+              y1 = fma(lx[m], px[j], y1);
+              y0 = fma(ly[j], py[m], y0);
+              y1 = fma(ly[m], py[j], y1);
               z += w[j] - w[m];
             }
           v[3 * q] = x0 - x1;
@@ -425,7 +428,7 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
           v[3 * q + 2] = z;
         }
         v[12] = v[13] = v[14] = v[15] = 0;
-        const F x = warp_rs16(v, lane);
+        const A x = warp_rs16(v, lane);
         if (!(lane & 1u)) sacc[(warp * nst + k) * 16 + (lane >> 1)] += static_cast<double>(x) * (static_cast<double>(cs) * cs);
       }
       if (!(P.direct && k == 0)) __syncthreads();
@@ -622,8 +625,9 @@ template <typename C, int T> constexpr int fwd_minb() {
   // 128 threads (11 bits): complex64 5 CTAs an SM (100 registers), complex128 3 (168)
   return sizeof(C) == 8 ? (T >= 12 ? 2 : T == 11 ? 5 : 8) : (T >= 12 ? 1 : T == 11 ? 3 : 6);
 }
-template <typename C, int T> constexpr int adj_minb() {
-  return sizeof(C) == 8 ? (T >= 12 ? 2 : T == 11 ? 4 : 8) : (T >= 12 ? 1 : T == 11 ? 2 : 4);
+template <typename C, typename A, int T> constexpr int adj_minb() {
+  if (sizeof(A) < sizeof(double)) return T == 11 ? 4 : 0;
+  return T >= 12 ? 1 : T == 11 ? 2 : sizeof(C) == 16 || T == 10 ? 4 : 8;
 }
 
 int pass_threads(const FramePass& p) { return 1 << (p.t - 4); }
@@ -644,19 +648,25 @@ template <typename C> const void* fwd_kernel(const FramePass& p) {
     default: return reinterpret_cast<const void*>(&k_frame_fwd<C, 12, fwd_minb<C, 12>()>);
   }
 }
-template <typename C> const void* adj_kernel(const FramePass& p) {
+// Cotangent sums of states below 2^16 amplitudes are float64 from the product on,
+// as in the general reverse pass of that size; larger states sum in the run
+// precision, as the specialised passes do.
+template <typename C, typename A, int T> const void* adj_of() {
+  return reinterpret_cast<const void*>(&k_frame_adj<C, A, T, adj_minb<C, A, T>()>);
+}
+template <typename C> const void* adj_kernel(const FramePass& p, int nb) {
   switch (p.t) {
-    case 9: return reinterpret_cast<const void*>(&k_frame_adj<C, 9, adj_minb<C, 9>()>);
-    case 10: return reinterpret_cast<const void*>(&k_frame_adj<C, 10, adj_minb<C, 10>()>);
-    case 11: return reinterpret_cast<const void*>(&k_frame_adj<C, 11, adj_minb<C, 11>()>);
-    default: return reinterpret_cast<const void*>(&k_frame_adj<C, 12, adj_minb<C, 12>()>);
+    case 9: return adj_of<C, double, 9>();
+    case 10: return adj_of<C, double, 10>();
+    case 11: return nb < 16 ? adj_of<C, double, 11>() : adj_of<C, Real<C>, 11>();
+    default: return adj_of<C, double, 12>();  // whole states only
   }
 }
 
-template <typename C> int upload_shapes(const FramePlan& fp, FrameDev* d) {
+template <typename C> int upload_shapes(const FramePlan& fp, int nb, FrameDev* d) {
   for (const FramePass& p : fp.passes) {
     for (int adj = 0; adj < 2; ++adj) {
-      const void* k = adj ? adj_kernel<C>(p) : fwd_kernel<C>(p);
+      const void* k = adj ? adj_kernel<C>(p, nb) : fwd_kernel<C>(p);
       const size_t smem = adj ? adj_smem<C>(p) : fwd_smem<C>(p);
       JQ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
       int n = 0;
@@ -718,7 +728,7 @@ int adjoint_t(const jq_plan* plan, const FrameDev& d, const C* psi_in, C* psi, C
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = pdl && i + 1 < fp.passes.size() ? 1 : 0;
-    JQ_CUDA(cudaLaunchKernelExC(&cfg, adj_kernel<C>(p), args));
+    JQ_CUDA(cudaLaunchKernelExC(&cfg, adj_kernel<C>(p, plan->n_bits), args));
   }
   return JQ_OK;
 }
@@ -741,7 +751,7 @@ int frame_upload(const jq_plan* plan, FrameDev* d) {
   if (!fp.on) return JQ_OK;
   const int rc = frame_tables(fp, d);
   if (rc) return rc;
-  return plan->dtype == JQ_C64 ? upload_shapes<float2>(fp, d) : upload_shapes<double2>(fp, d);
+  return plan->dtype == JQ_C64 ? upload_shapes<float2>(fp, plan->n_bits, d) : upload_shapes<double2>(fp, plan->n_bits, d);
 }
 
 void frame_free(FrameDev* d) {

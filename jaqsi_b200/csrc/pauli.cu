@@ -102,18 +102,18 @@ template <int S, bool PAIR, typename F> __device__ __forceinline__ void apply_mt
   }
 }
 // g[4 (i - 1) + j] = sum of l (entry i of the wire) times x (entry j), i = 1..3
-template <int S, bool PAIR, typename F>
-__device__ __forceinline__ void outer_sum(const F (&l)[16], const F (&x)[16], F (&g)[16]) {
+template <int S, bool PAIR, typename F, typename A>
+__device__ __forceinline__ void outer_sum(const F (&l)[16], const F (&x)[16], A (&g)[16]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      F a = 0;
+      A a = 0;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int b = S == 1 ? 4 * q : q;
-        const F y = x[b + j * S];
-        a = fma(l[b + (i + 1) * S], PAIR && q == 3 && odd_entry(4 * i + j) ? -y : y, a);
+        const A y = x[b + j * S];
+        a = fma(static_cast<A>(l[b + (i + 1) * S]), PAIR && q == 3 && odd_entry(4 * i + j) ? -y : y, a);
       }
       g[4 * i + j] = a;
     }
@@ -278,11 +278,11 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
 // One reverse pass: the input of every stage is kept in shared memory by a
 // forward walk over the tile; backwards, each wire's cotangent (entries of lambda
 // after its matrix times entries of the values before it, the other wire's matrix
-// on one side) is summed, per tile and warp in the run precision, in float64
-// across tiles, and lambda goes through the transposed matrices.
+// on one side) is summed, in type A in a thread and a warp, in float64 across warps
+// and tiles, and lambda goes through the transposed matrices.
 // Not launched ahead of the previous pass: two of these on an SM at once take each
 // other's L2 (12 qubits 7.08 instead of 6.72 ms).
-template <typename F, int T, int MINB>
+template <typename F, typename A, int T, int MINB>
 __global__ void __launch_bounds__(1 << (T - 4), MINB)
     k_pauli_bwd(const F* __restrict__ xin, F* __restrict__ lam, const PassArg P, const FrameStage* __restrict__ stages,
                 const F* __restrict__ bmat, int64_t bstride, double* __restrict__ gacc, int64_t gstride, int batch) {
@@ -366,8 +366,8 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
       for (int j = 0; j < 16; ++j) l[j] = lds<F>(lt + a[j]);
       double* acc = sacc + (warp * nst + k) * 32;
       const bool wa = gacc && st[k].gate[0] >= 0, wb = gacc && st[k].ng > 1 && st[k].gate[2] >= 0;
-      auto add = [&](double* to, F (&g)[16]) {
-        const F t = warp_rs16(g, lane);
+      auto add = [&](double* to, A (&g)[16]) {
+        const A t = warp_rs16(g, lane);
         if (!(lane & 1u)) to[lane >> 1] += static_cast<double>(t);
       };
       F x[16];
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
       }
       if (st[k].ng == 2) {
         const uint32_t p = y_parity(g0);
-        F g[16];
+        A g[16];
         if (wb) {
           F y[16];
           load12(tb.m[0], c);
@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
       } else {
         column_signs(l, g0, st[k]);
         if (wa) {
-          F g[16];
+          A g[16];
           column_signs(x, g0, st[k]);
           outer_sum<1, false>(l, x, g);
           add(acc, g);
@@ -599,7 +599,9 @@ __global__ void k_pauli_seed(F* __restrict__ lam, int nb, const PauliObs* __rest
 }
 
 template <typename F, int T> constexpr int fwd_ctas() { return sizeof(F) == 4 ? (T == 11 ? 8 : 16) : (T == 11 ? 5 : 10); }
-template <typename F, int T> constexpr int bwd_ctas() { return sizeof(F) == 4 ? (T == 11 ? 4 : 8) : (T == 11 ? 2 : 4); }
+template <typename F, typename A, int T> constexpr int bwd_ctas() {
+  return sizeof(A) == 4 ? 4 : sizeof(F) == 4 ? (T == 11 ? 3 : 6) : (T == 11 ? 2 : 4);
+}
 
 template <typename F> size_t fwd_smem(const FramePass& p) {
   return (static_cast<size_t>(2) << p.t) * sizeof(F) + pauli_tables<F>(p.nst, 1 << (p.t - 4));
@@ -613,15 +615,21 @@ template <typename F> const void* fwd_kernel(const FramePass& p) {
   return p.t == 10 ? reinterpret_cast<const void*>(&k_pauli_fwd<F, 10, fwd_ctas<F, 10>()>)
                    : reinterpret_cast<const void*>(&k_pauli_fwd<F, 11, fwd_ctas<F, 11>()>);
 }
-template <typename F> const void* bwd_kernel(const FramePass& p) {
-  return p.t == 10 ? reinterpret_cast<const void*>(&k_pauli_bwd<F, 10, bwd_ctas<F, 10>()>)
-                   : reinterpret_cast<const void*>(&k_pauli_bwd<F, 11, bwd_ctas<F, 11>()>);
+// Cotangent sums below 2^16 coefficients (seven qubits) are float64 from the product
+// on, as in the general reverse pass of that size; larger ones are summed in the
+// run precision, as in the specialised reverse steps.
+template <typename F, typename A, int T> const void* bwd_of() {
+  return reinterpret_cast<const void*>(&k_pauli_bwd<F, A, T, bwd_ctas<F, A, T>()>);
+}
+template <typename F> const void* bwd_kernel(const FramePass& p, int nb) {
+  if (p.t == 10) return bwd_of<F, double, 10>();  // five qubits
+  return nb < 16 ? bwd_of<F, double, 11>() : bwd_of<F, F, 11>();
 }
 
-template <typename F> int upload_shapes(const FramePlan& fp, FrameDev* d) {
+template <typename F> int upload_shapes(const FramePlan& fp, int nb, FrameDev* d) {
   for (const FramePass& p : fp.passes)
     for (int rev = 0; rev < 2; ++rev) {
-      const void* k = rev ? bwd_kernel<F>(p) : fwd_kernel<F>(p);
+      const void* k = rev ? bwd_kernel<F>(p, nb) : fwd_kernel<F>(p);
       JQ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
       int n = 0;
       JQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, 1 << (p.t - 4), rev ? bwd_smem<F>(p) : fwd_smem<F>(p)));
@@ -736,7 +744,7 @@ int backward_t(const jq_plan* plan, const FrameDev& d, const DeviceTables& T, in
       int64_t gs = gstride;
       void* args[] = {&xin, &lam, &a, &sp, &bmat, &bs, &gacc, &gs, &batch};
       JQ_CUDA(cudaLaunchKernel(
-          bwd_kernel<F>(fpz),
+          bwd_kernel<F>(fpz, plan->n_bits),
           dim3(static_cast<unsigned>(std::min<int64_t>(ntiles, static_cast<int64_t>(sms) * d.adj_ctas[static_cast<size_t>(p)]))),
           dim3(1u << (fpz.t - 4)), args, bwd_smem<F>(fpz), st));
     }
@@ -759,7 +767,7 @@ int pauli_upload(const jq_plan* plan, FrameDev* d) {
   if (!fp.on) return JQ_OK;
   int rc = frame_tables(fp, d);
   if (rc) return rc;
-  return plan->dtype == JQ_C64 ? upload_shapes<float>(fp, d) : upload_shapes<double>(fp, d);
+  return plan->dtype == JQ_C64 ? upload_shapes<float>(fp, plan->n_bits, d) : upload_shapes<double>(fp, plan->n_bits, d);
 }
 
 int pauli_forward(const jq_plan* plan, const DeviceTables& T, int batch, const double* angles, void* state, void* bmat,

@@ -11,8 +11,6 @@ import pytest
 import torch
 
 import jaqsi_b200 as jq
-from jaqsi_b200 import _lib as L
-from jaqsi_b200 import simulation as sim
 
 pytestmark = pytest.mark.gpu
 TOL = {torch.complex64: 1e-5, torch.complex128: 1e-10}
@@ -41,3 +39,54 @@ def test_noisy_values_of_an_angle_that_is_not_finite(n, bad, gate, dtype):
     assert torch.isnan(ev[1]).all() and torch.isnan(params.grad[1]).all()
     assert torch.isfinite(ev[[0, 2]]).all() and torch.isfinite(params.grad[[0, 2]]).all()
     assert torch.equal(ev[0], ev[2])
+
+
+@pytest.mark.parametrize("n", [9, 10, 11, 12, 13, 15])
+def test_frame_cotangent_sums_of_small_states_are_float64(n):
+    """Complex64 states below 2^16 amplitudes.  Wire a starts in |+> and has no gate,
+    the others are turned into |+>, amplitudes exact but for a factor common to
+    all.  Where z_a = 1 the words z_x z_y (1 + z_a) / 2 leave every gradient zero in
+    terms of size 1; where z_a = -1, 2^-28 z_w (1 - z_a) / 2 has terms of size 2^-28,
+    which float32 sums over both lose and float64 sums hold to 2^-24."""
+    rng = np.random.default_rng(n)
+    parity = jq.build_parity_observable
+    for _ in range(100):
+        a, x, y, w = (int(v) for v in rng.choice(n, 4, replace=False))
+        script = jq.Script(lambda p: [jq.RY(p[k], wires=k) for k in range(n) if k != a] and None, n_qubits=n)
+        start = torch.zeros(2**n, dtype=torch.complex64)
+        start[0] = start[1 << (n - 1 - a)] = 0.5**0.5
+        obs = [parity([x, y]), parity([a, x, y]), jq.PauliZ(w), parity([a, w])]
+        params = torch.full((n,), np.pi / 2, dtype=torch.float64, requires_grad=True)
+        ev = script.execute("expval", obs, args=(params,), initial_state=start, dtype=torch.complex64)
+        ct = torch.tensor([0.5, 0.5, 2.0**-29, -(2.0**-29)], device=ev.device, dtype=torch.float64)
+        (ev.to(torch.float64) @ ct).backward()
+        want = np.zeros(n)
+        want[w] = -(2.0**-29)
+        np.testing.assert_allclose(params.grad.numpy(), want, atol=TOL[torch.complex64] * 2.0**-29, rtol=0,
+                                   err_msg=f"{a} {x} {y} {w}")
+
+
+@pytest.mark.parametrize("n", [5, 6, 7])
+def test_pauli_cotangent_sums_of_small_states_are_float64(n):
+    """Complex64 coefficients below 2^16: wires b, c, d stay in |0>, so that z_w z_b -
+    z_w z_c + 2^-28 z_w z_d has the gradient of 2^-28 z_w, whose terms in a sum
+    over coefficients are 1, -1 and 2^-28."""
+    parity = jq.build_parity_observable
+
+    def circuit(p):
+        jq.RY(p[0], wires=0)
+        jq.AmplitudeDamping(0.1, wires=0)
+
+    script = jq.Script(circuit, n_qubits=n)
+    want = -(2.0**-28) * 0.9 * np.sin(0.7)
+    for b in range(1, n):
+        for c in range(1, n):
+            for d in range(1, n):
+                if len({b, c, d}) < 3:
+                    continue
+                p = torch.tensor([0.7], dtype=torch.float64, requires_grad=True)
+                ev = script.execute("expval", [parity([0, b]), parity([0, c]), parity([0, d])], args=(p,),
+                                    dtype=torch.complex64)
+                ct = torch.tensor([1.0, -1.0, 2.0**-28], device=ev.device, dtype=torch.float64)
+                (ev.to(torch.float64) @ ct).backward()
+                np.testing.assert_allclose(p.grad.numpy(), [want], rtol=TOL[torch.complex64], err_msg=f"{b} {c} {d}")
