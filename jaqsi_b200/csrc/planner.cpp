@@ -204,6 +204,23 @@ bool pauli_map(const std::vector<cd>& s) {
   return true;
 }
 
+// Whether a frame plan costs no more than the specialised passes, of which a stage
+// holds gates that need not commute.  In units of a general gate a frame stage
+// costs the same below 20 qubits (both are latency) and 2.5 gates from there on, a
+// pass 2 in either, a call 4 more without the frame (its start state is written and
+// read).  Measured forward, general / frame (us): 24 qubits complex64, 12 layers on
+// two wires (24 gates, 12 stages) 224 / 315, on three (36, 12) 323 / 315, ring of 4
+// layers (96, 27) 830 / 633; one gate a stage 224 / 514 (24), 81 / 160 (22), 40 / 64
+// (20), 33 / 38 (16); complex128 two wires 365 / 535 (24), 50 / 57 (20), 35 / 32 (16).
+// Below 2^16 amplitudes the alternative is an interpreter: one gate a stage 45 / 44 at
+// 12 qubits complex64 and 54 / 56 in complex128, everything else is further apart.
+bool frame_pays(const FramePlan& f, size_t general_passes, int nb) {
+  if (nb < 16) return true;
+  const double stage = nb >= 20 ? 2.5 : 1.0;
+  return stage * static_cast<double>(f.stages.size()) + 2.0 * static_cast<double>(f.passes.size()) <=
+         static_cast<double>(f.gates.size()) + 2.0 * static_cast<double>(general_passes) + 4.0;
+}
+
 bool is_unitary2(const std::vector<cd>& m) {
   if (m.size() != 4) return false;
   for (int i = 0; i < 2; ++i)
@@ -970,7 +987,10 @@ int build_plan(const jq_op* ops, int n_ops, const jq_obs* obs, int n_obs, int n_
     // 20 qubits 3.87 against 3.63 ms.
     const int ft = nb <= kFrameMaxT ? nb : 11;
     const int fc = dtype == JQ_C64 && nb >= 24 ? 4 : 3;
-    if (ok && frame_schedule(fops, nb, ft, fc, dtype == JQ_C64 ? 8 : 16, ft == nb ? kFrameMaxStages : kFrameBallot, &zt, &zsign, &plan->frame)) {
+    FramePlan frame;
+    if (ok && frame_schedule(fops, nb, ft, fc, dtype == JQ_C64 ? 8 : 16, ft == nb ? kFrameMaxStages : kFrameBallot, &zt, &zsign, &frame) &&
+        (!plan->jit || frame_pays(frame, plan->fwd.passes.size(), nb))) {
+      plan->frame = std::move(frame);
       plan->frame_obs = plan->obs;
       for (int i = 0; i < n_obs; ++i) {
         plan->frame_obs[i].z_mask = zt[i];
