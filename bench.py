@@ -284,7 +284,7 @@ class Direct:
         self.out = torch.empty((batch, max(plan.n_obs, 1)), dtype=torch.float64, device=dev)
         self.ct = torch.ones((batch, max(plan.n_obs, 1)), dtype=torch.float64, device=dev)
         self.ga = torch.empty((batch, max(plan.n_angles, 1)), dtype=torch.float64, device=dev)
-        mode = {None: 0, "adjoint": 1, "backward": 2}[grad]
+        mode = {None: 0, "adjoint": 1, "backward": 3}[grad]
         self.wsb = max(plan.workspace_bytes(batch, 0), plan.workspace_bytes(batch, mode))
         self.ws = torch.empty(max(self.wsb, 1), dtype=torch.uint8, device=dev)
         self.stream = torch.cuda.current_stream()

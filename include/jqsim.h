@@ -214,7 +214,10 @@ JQ_API int jq_plan_block_passes(const jq_plan* plan, int which, int32_t* block_p
 JQ_API size_t jq_plan_jit_source(const jq_plan* plan, char* buf, size_t n);
 
 /* Device workspace (bytes) for `batch` instances: with_grad 0 sizes
- * jq_forward, 1 sizes jq_adjoint, 2 sizes jq_backward. */
+ * jq_forward, 1 sizes jq_adjoint, 2 sizes jq_backward (the least it takes), 3
+ * sizes jq_backward with room to keep more of the states it otherwise recomputes:
+ * a plan on Pauli coefficients (jq_tune.expval_only = 2) uses whatever it is
+ * given beyond the least; all others take the same in 2 and 3. */
 JQ_API size_t jq_workspace_bytes(const jq_plan* plan, int batch, int out_type,
                           int with_grad);
 

@@ -2225,7 +2225,9 @@ struct WsLayout {
   int64_t n_ckpt = 0, seg_len = 0;
 };
 
-WsLayout layout(const jq_plan* plan, int batch, int mode_grad /*0 fwd, 1 adjoint, 2 ckpt*/) {
+// mode_grad: 0 forward, 1 adjoint, 2 checkpointed reverse pass, 3 the same with room
+// for more pass inputs of a plan on Pauli coefficients
+WsLayout layout(const jq_plan* plan, int batch, int mode_grad) {
   WsLayout L;
   const size_t elem = plan->dtype == JQ_C64 ? 8 : 16;
   const size_t state = static_cast<size_t>(plan->state_elems) * elem * batch;
@@ -2245,7 +2247,7 @@ WsLayout layout(const jq_plan* plan, int batch, int mode_grad /*0 fwd, 1 adjoint
     L.psi = off;
     off += align256(state);
   }
-  if (mode_grad == 2) {
+  if (mode_grad >= 2) {
     const int64_t P = static_cast<int64_t>(plan->fwd.passes.size());
     int64_t S = plan->ckpt_stride > 0 ? plan->ckpt_stride : static_cast<int64_t>(std::ceil(std::sqrt(static_cast<double>(std::max<int64_t>(P, 1)))));
     S = std::max<int64_t>(1, S);
@@ -2258,14 +2260,17 @@ WsLayout layout(const jq_plan* plan, int batch, int mode_grad /*0 fwd, 1 adjoint
     L.seg = off;
     off += align256(state) * static_cast<size_t>(S);
     if (plan->pauli.on) {
-      // half-size states: every pass input while that takes 256 MB or half as much
-      // again as the general passes at most, two levels of checkpoints at least
+      // half-size states: two levels of checkpoints, which fit into what the general
+      // passes take but for circuits of few of those; with room, every pass input
+      // while that takes 256 MB or half as much again at most (the general passes of
+      // 15 qubits and 8 layers take 146 GB in complex64)
       const size_t half = align256(state / 2);
       const int64_t Q = static_cast<int64_t>(plan->pauli.passes.size());
       int64_t two = Q;
       for (int64_t s = 1; s < Q; ++s) two = std::min(two, (Q + s - 1) / s + s);
       const size_t all = static_cast<size_t>(Q) * half;
-      const int64_t need = all <= (size_t{256} << 20) || L.work + all <= off + off / 2 ? Q : two;
+      const bool keep = mode_grad == 3 && (all <= (size_t{256} << 20) || L.work + all <= off + off / 2);
+      const int64_t need = keep ? Q : two;
       off = std::max(off, L.work + half * static_cast<size_t>(std::max<int64_t>(need, 1)));
     }
   }
@@ -2730,10 +2735,10 @@ int backward_impl(const jq_plan* plan, int batch, const double* angles, const vo
   }
   if (pauli) {
     char* wp = static_cast<char*>(ws);
-    // the coefficients take half a state; everything behind lambda but the
-    // cotangents holds pass inputs
+    // the coefficients take half a state; all of the caller's workspace behind lambda
+    // but the cotangents holds pass inputs
     const size_t half = align256(static_cast<size_t>(plan->state_elems) * sizeof(R) * batch);
-    const int64_t n_slots = static_cast<int64_t>((L.total - L.work) / half);
+    const int64_t n_slots = static_cast<int64_t>((ws_bytes - L.work) / half);
     if (grad_mats && plan->n_mats > 0)
       JQ_CUDA(cudaMemsetAsync(grad_mats, 0, 16 * static_cast<size_t>(plan->n_mats) * batch, st));
     return pauli_backward(plan, *T, batch, angles, wp + L.bmat, reinterpret_cast<double*>(wp + L.gacc), wp + L.lam,
@@ -3051,7 +3056,7 @@ size_t jq_workspace_bytes(const jq_plan* plan, int batch, int out_type, int with
   if (!plan || batch < 1) return 0;
   int mode = 0;
   if (with_grad == 1) mode = 1;       // jq_adjoint
-  else if (with_grad == 2) mode = 2;  // jq_backward
+  else if (with_grad == 2 || with_grad == 3) mode = with_grad;  // jq_backward
   return layout(plan, batch, mode).total;
 }
 

@@ -681,6 +681,10 @@ def _grad_launch(plan: Plan, out_type: int, batch: int, init_batched: int, need,
     return tuple(torch.cat(p) if p[0].numel() else p[0] for p in zip(*parts))
 
 
+def _workspace(nbytes: int, dev) -> torch.Tensor:
+    return torch.empty(max(nbytes, 1), dtype=torch.uint8, device=dev)
+
+
 def _grad_launch_whole(plan: Plan, out_type: int, batch: int, init_batched: int, need, angles, mats, init, state, g):
     dev = state.device
     lib = plan._lib
@@ -694,8 +698,14 @@ def _grad_launch_whole(plan: Plan, out_type: int, batch: int, init_batched: int,
     gdim = plan.state_elems if init_batched & _INIT_DENSITY else 1 << plan.n_qubits
     gi = torch.empty((batch, gdim), dtype=plan.cdtype, device=dev) if need[2] else None
     use_adjoint = plan.mode == L.JQ_STATEVECTOR and plan.unitary
-    wsb = plan.workspace_bytes(batch, 1 if use_adjoint else 2)
-    ws = torch.empty(max(wsb, 1), dtype=torch.uint8, device=dev)
+    if use_adjoint:
+        ws = _workspace(plan.workspace_bytes(batch, 1), dev)
+    else:
+        try:
+            ws = _workspace(plan.workspace_bytes(batch, 3), dev)
+        except torch.OutOfMemoryError:
+            ws = _workspace(plan.workspace_bytes(batch, 2), dev)
+    wsb = ws.numel()
     if use_adjoint:
         L.check(
             lib.jq_adjoint(

@@ -72,3 +72,29 @@ def test_circuits_on_every_wire_run_in_the_frame(family, dtype):
         for layers in (2, 5, 20):
             a = np.full((layers, n, 3), 0.1)
             assert _own(lambda: family(n, layers, a), n, [jq.PauliZ(w) for w in range(n)], dtype), (n, layers)
+
+
+def _noisy(n, layers):
+    return lambda: wl.noisy_ansatz(n, layers, np.full((layers, n, 3), 0.1), 0.01, 0.005)
+
+
+def _workspaces(circuit, n, dtype, batch, with_grad):
+    with jq.recording() as tape:
+        circuit()
+    lw = sim.lower_tape(tape, n)
+    specs, _ = sim._lower_obs([jq.PauliZ(0)], n)
+    return [sim.Plan(lw.statics, specs, n, L.JQ_DENSITY, dtype, {"expval_only": e}).workspace_bytes(batch, with_grad)
+            for e in (1, 2)]
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("n,layers,batch", [(7, 40, 1), (9, 20, 3), (12, 8, 1), (15, 2, 1), (15, 8, 1)])
+def test_reverse_call_on_pauli_coefficients_needs_no_more_than_the_general_one(n, layers, batch, dtype):
+    """The least jq_backward takes is what the general passes take: 15 qubits with 8
+    layers fit one GPU in complex64 (17 states of 8.6 GB) as they did without the
+    coefficients.  With room for more it is half as much again at most."""
+    general, own = _workspaces(_noisy(n, layers), n, dtype, batch, 2)
+    assert own == general
+    roomy = _workspaces(_noisy(n, layers), n, dtype, batch, 3)
+    assert roomy[0] == general
+    assert general <= roomy[1] <= max(1.5 * general, general + (256 << 20))

@@ -11,6 +11,9 @@ import pytest
 import torch
 
 import jaqsi_b200 as jq
+from jaqsi_b200 import _lib as L
+from jaqsi_b200 import simulation as sim
+from jaqsi_b200 import workloads as wl
 
 pytestmark = pytest.mark.gpu
 TOL = {torch.complex64: 1e-5, torch.complex128: 1e-10}
@@ -90,3 +93,67 @@ def test_pauli_cotangent_sums_of_small_states_are_float64(n):
                 ct = torch.tensor([1.0, -1.0, 2.0**-28], device=ev.device, dtype=torch.float64)
                 (ev.to(torch.float64) @ ct).backward()
                 np.testing.assert_allclose(p.grad.numpy(), [want], rtol=TOL[torch.complex64], err_msg=f"{b} {c} {d}")
+
+
+def _noisy_plans(n, layers, noise, obs, dtype):
+    """A noisy circuit on the general passes and on Pauli coefficients."""
+    with jq.recording() as tape:
+        wl.noisy_ansatz(n, layers, np.zeros((layers, n, 3)), noise, noise)
+    lw = sim.lower_tape(tape, n)
+    specs, _ = sim._lower_obs(obs, n)
+    statics = [st[:10] + (1,) + st[11:] if st[3] >= 0 else st for st in lw.statics]  # every angle trainable
+    return [sim.Plan(statics, specs, n, L.JQ_DENSITY, dtype, {"expval_only": e}) for e in (1, 2)]
+
+
+def _backward(plan, angles, ct, with_grad):
+    batch = angles.shape[0]
+    grad = torch.empty((batch, plan.n_angles), dtype=torch.float64, device="cuda")
+    ws = torch.full((plan.workspace_bytes(batch, with_grad),), 255, dtype=torch.uint8, device="cuda")  # NaNs
+    L.check(plan._lib.jq_backward(plan.handle, batch, sim._ptr(angles), None, None, 0, L.JQ_OUT_EXPVAL, sim._ptr(ct),
+                                  None, sim._ptr(grad), None, None, sim._ptr(ws), ws.numel(), sim._stream()))
+    return grad.cpu().numpy()
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("n,layers,batch", [(6, 40, 2), (6, 80, 1), (7, 40, 1), (7, 60, 2), (9, 20, 1)])
+def test_segments_of_the_pauli_reverse_pass(n, layers, batch, dtype):
+    """More passes than the least workspace holds states: the inputs of a segment are
+    recomputed from its checkpoint.  Every gradient, against the call that keeps
+    all inputs (the same kernels on the same values: only the order of float64
+    additions differs) and against the general passes."""
+    rng = np.random.default_rng(n * layers)
+    obs = [jq.PauliZ(0), jq.PauliX(n - 1), jq.PauliZ(2)]
+    general, own = _noisy_plans(n, layers, 0.001, obs, dtype)
+    half = own.state_elems * batch * (4 if dtype == torch.complex64 else 8)
+    assert own.info["n_passes_fwd"] > own.workspace_bytes(batch, 2) // half
+    angles = torch.tensor(rng.uniform(0, 2 * np.pi, (batch, own.n_angles)), device="cuda")
+    ct = torch.tensor(rng.normal(size=(batch, len(obs))), device="cuda")
+    least, roomy = _backward(own, angles, ct, 2), _backward(own, angles, ct, 3)
+    np.testing.assert_allclose(least, roomy, atol=1e-13, rtol=0)
+    want = _backward(general, angles, ct, 2)
+    np.testing.assert_allclose(least, want, atol=TOL[dtype] * np.abs(ct.cpu().numpy()).sum(1).max() * n, rtol=0)
+    assert np.abs(want).max() > 1e-3
+
+
+def test_reverse_call_takes_less_where_memory_is_short(monkeypatch):
+    """The larger workspace does not fit: the call runs in the smaller one."""
+    n, layers = 7, 40
+    script = jq.Script(lambda a: wl.noisy_ansatz(n, layers, a, 0.001, 0.001), n_qubits=n)
+    base = torch.rand(layers, n, 3, generator=torch.Generator().manual_seed(3), dtype=torch.float64) * 6
+    given, make = [], sim._workspace
+
+    def limited(nbytes, dev):
+        given.append(nbytes)
+        if len(given) == 1:
+            raise torch.OutOfMemoryError("test")
+        return make(nbytes, dev)
+
+    grads = []
+    for patched in (False, True):
+        if patched:
+            monkeypatch.setattr(sim, "_workspace", limited)
+        p = base.clone().requires_grad_(True)
+        script.execute("expval", [jq.PauliZ(0)], args=(p,)).sum().backward()
+        grads.append(p.grad)
+    assert len(given) == 2 and given[1] < given[0]
+    torch.testing.assert_close(grads[0], grads[1], atol=1e-13, rtol=0)
