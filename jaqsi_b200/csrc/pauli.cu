@@ -192,7 +192,7 @@ template <typename F> __host__ __device__ constexpr size_t pauli_tables(int nst,
 template <typename F, int T, int MINB>
 __global__ void __launch_bounds__(1 << (T - 4), MINB)
     k_pauli_fwd(const F* in, F* out, const PassArg P, const FrameStage* __restrict__ stages, const F* __restrict__ bmat,
-                int64_t bstride, int batch, int rev) {
+                int64_t bstride, int batch, int rev, int first) {
   constexpr int LT = T - 4, NT = 1 << LT;
   constexpr uint32_t TB = sizeof(F) << T;
   const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
   uint32_t* tg = gso + 16 * P.nst;
   uint16_t* tbs = reinterpret_cast<uint16_t*>(tg + NT * P.nst);
   const uint32_t tid = threadIdx.x, lane = tid & 31u;
-  asm volatile("griddepcontrol.launch_dependents;");
+  if (!first) asm volatile("griddepcontrol.launch_dependents;");
   const FrameStage* st = stages + P.st0;
   const int nst = P.nst;
   pauli_setup<LT>(st, nst, tbs, soff, gso, tg);
@@ -220,9 +220,11 @@ __global__ void __launch_bounds__(1 << (T - 4), MINB)
     const F* src = in + ((tl >> P.nouter) << P.nb);
     copy.each(P, rep_of(tl), dst, [&](uint32_t a, uint32_t b) { cp_async16(sbase + b, src + a); });
   };
-  // the first pass of a call follows prep in plain stream order: the matrices need
-  // no wait, the states do
+  // The first pass of a call may start before prep has written the matrices: it waits,
+  // and only then lets the second start.  From there on the matrices need no
+  // wait, the states do.
   int64_t last = -1;
+  if (first) asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;" ::: "memory");
   if (blockIdx.x < ntiles) {
     last = static_cast<int64_t>(blockIdx.x) >> P.nouter;
     pass_tables<F, LT>(st, nst, bmat + last * bstride, tab);
@@ -656,8 +658,8 @@ int pass_fwd(const jq_plan* plan, const FrameDev& d, size_t i, const F* in, F* o
   cfg.numAttrs = pdl ? 1 : 0;
   const FrameStage* sp = d.stages;
   int64_t bs = 2 * plan->bmat_stride;
-  int rev = static_cast<int>(i & 1);
-  void* args[] = {&in, &out, &a, &sp, &bmat, &bs, &batch, &rev};
+  int rev = static_cast<int>(i & 1), first = i == 0;
+  void* args[] = {&in, &out, &a, &sp, &bmat, &bs, &batch, &rev, &first};
   JQ_CUDA(cudaLaunchKernelExC(&cfg, fwd_kernel<F>(p), args));
   return JQ_OK;
 }
@@ -686,7 +688,7 @@ int forward_t(const jq_plan* plan, const FrameDev& d, const DeviceTables& T, int
   if (rc) return rc;
   const bool pdl = pdl_on(st);
   for (size_t i = 0; i < plan->pauli.passes.size(); ++i)
-    if ((rc = pass_fwd<F>(plan, d, i, s, s, batch, bmat, sms, st, pdl && i > 0))) return rc;
+    if ((rc = pass_fwd<F>(plan, d, i, s, s, batch, bmat, sms, st, pdl))) return rc;
   const int no = static_cast<int>(plan->pauli_obs.size());
   k_pauli_expval<F><<<blocks_for(static_cast<int64_t>(no) * batch, 128), 128, 0, st>>>(
       s, plan->n_bits, static_cast<const PauliObs*>(T.pauli_obs), no, batch, out);
@@ -718,7 +720,7 @@ int backward_t(const jq_plan* plan, const FrameDev& d, const DeviceTables& T, in
     for (int64_t c = 0; c + 1 < nck; ++c)  // checkpoint c + 1 from c, through the segment's buffer
       for (int64_t p = c * S; p < (c + 1) * S; ++p)
         if ((rc = pass_fwd<F>(plan, d, static_cast<size_t>(p), p == c * S ? slot(c) : seg(0),
-                              p + 1 == (c + 1) * S ? slot(c + 1) : seg(0), batch, bmat, sms, st, pdl && p > 0)))
+                              p + 1 == (c + 1) * S ? slot(c + 1) : seg(0), batch, bmat, sms, st, pdl)))
           return rc;
   JQ_CUDA(cudaMemsetAsync(lam, 0, bytes, st));
   const int no = static_cast<int>(plan->pauli_obs.size());
@@ -732,8 +734,7 @@ int backward_t(const jq_plan* plan, const FrameDev& d, const DeviceTables& T, in
     const int64_t p0 = c * S, p1 = std::min(P, p0 + S);
     auto input = [&](int64_t p) { return nck > 0 ? (p == p0 ? slot(c) : seg(p - p0 - 1)) : slot(p); };
     for (int64_t p = p0; p + 1 < p1; ++p)
-      if ((rc = pass_fwd<F>(plan, d, static_cast<size_t>(p), input(p), input(p + 1), batch, bmat, sms, st, pdl && p > 0)))
-        return rc;
+      if ((rc = pass_fwd<F>(plan, d, static_cast<size_t>(p), input(p), input(p + 1), batch, bmat, sms, st, pdl))) return rc;
     for (int64_t p = p1 - 1; p >= p0 && want; --p) {
       const FramePass& fpz = fp.passes[static_cast<size_t>(p)];
       PassArg a = pass_arg(fpz, plan->n_bits, true);
