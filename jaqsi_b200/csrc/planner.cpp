@@ -184,9 +184,16 @@ bool pauli_perm(const HostBlock& hb, int n, FrameOp* f) {
   return true;
 }
 
+// How far a constant may be from unitary, or from keeping trace and Hermiticity, in
+// a representation that takes it as exact: a few units in the last place, as
+// gates and channels that were computed in float64 are (2e-15 over random Kraus
+// sets, QR factors and exponentials), so that a circuit of a thousand of them is
+// off by no more than its rounding.  complex64 runs round every matrix to 6e-8.
+double exact_within(int dtype) { return dtype == JQ_C64 ? 1e-12 : 4e-15; }
+
 // A constant one-qubit superoperator on (ket, bra) that keeps the trace and
 // Hermiticity: a real matrix on Pauli coefficients with first row (1, 0, 0, 0).
-bool pauli_map(const std::vector<cd>& s) {
+bool pauli_map(const std::vector<cd>& s, double tol) {
   if (s.size() != 16) return false;
   const cd i1(0, 1);
   const cd q[4][4] = {{1, 0, 0, 1}, {0, 1, 1, 0}, {1, 0, 0, -1}, {0, -i1, i1, 0}};  // I, X, Z, Y row-major
@@ -196,9 +203,9 @@ bool pauli_map(const std::vector<cd>& s) {
       x[r] = 0;
       for (int t = 0; t < 4; ++t) x[r] += s[4 * r + t] * q[c][t];
     }
-    if (std::abs(x[0] + x[3] - cd(c == 0 ? 2 : 0, 0)) > 1e-12) return false;
-    if (std::abs((x[1] + x[2]).imag()) > 1e-12 || std::abs((x[0] - x[3]).imag()) > 1e-12 ||
-        std::abs((x[2] - x[1]).real()) > 1e-12)
+    if (std::abs(x[0] + x[3] - cd(c == 0 ? 2 : 0, 0)) > tol) return false;
+    if (std::abs((x[1] + x[2]).imag()) > tol || std::abs((x[0] - x[3]).imag()) > tol ||
+        std::abs((x[2] - x[1]).real()) > tol)
       return false;
   }
   return true;
@@ -221,12 +228,12 @@ bool frame_pays(const FramePlan& f, size_t general_passes, int nb) {
          static_cast<double>(f.gates.size()) + 2.0 * static_cast<double>(general_passes) + 4.0;
 }
 
-bool is_unitary2(const std::vector<cd>& m) {
+bool is_unitary2(const std::vector<cd>& m, double tol) {
   if (m.size() != 4) return false;
   for (int i = 0; i < 2; ++i)
     for (int j = 0; j < 2; ++j) {
       const cd v = m[i] * std::conj(m[j]) + m[2 + i] * std::conj(m[2 + j]);
-      if (std::abs(v - cd(i == j ? 1 : 0, 0)) > 1e-12) return false;
+      if (std::abs(v - cd(i == j ? 1 : 0, 0)) > tol) return false;
     }
   return true;
 }
@@ -966,7 +973,7 @@ int build_plan(const jq_op* ops, int n_ops, const jq_obs* obs, int n_obs, int n_
         for (int pi : hb.prims) {
           const HostPrim& p = prims[pi];
           if (!ok) break;
-          if (p.form == PF_CONST) { ok = is_unitary2(p.cmat); continue; }
+          if (p.form == PF_CONST) { ok = is_unitary2(p.cmat, exact_within(dtype)); continue; }
           const int kind = p.op >= 0 ? plan->ops[p.op].kind : -1;
           ok = p.form == PF_U && (kind == JQ_K_RX || kind == JQ_K_RY || kind == JQ_K_RZ || kind == JQ_K_ROT ||
                                   (kind == JQ_K_PAULIROT && (plan->ops[p.op].px | plan->ops[p.op].pz) != 0));
@@ -1022,7 +1029,7 @@ int build_plan(const jq_op* ops, int n_ops, const jq_obs* obs, int n_obs, int n_
         for (int pi : hb.prims) {
           const HostPrim& p = prims[pi];
           if (!ok) break;
-          if (p.form == PF_CONST) { ok = pauli_map(p.cmat); continue; }
+          if (p.form == PF_CONST) { ok = pauli_map(p.cmat, exact_within(dtype)); continue; }
           const int k = p.op >= 0 ? plan->ops[p.op].kind : -1;
           ok = p.form == PF_KRON && (k == JQ_K_RX || k == JQ_K_RY || k == JQ_K_RZ || k == JQ_K_ROT || k == JQ_K_CPHASE ||
                                      k == JQ_K_PAULIROT);

@@ -98,3 +98,87 @@ def test_reverse_call_on_pauli_coefficients_needs_no_more_than_the_general_one(n
     roomy = _workspaces(_noisy(n, layers), n, dtype, batch, 3)
     assert roomy[0] == general
     assert general <= roomy[1] <= max(1.5 * general, general + (256 << 20))
+
+
+@pytest.mark.parametrize("off", [4e-16, 1e-13, 1e-9])
+def test_constants_that_are_not_exact_keep_their_modulus(off):
+    """The frame divides by a gate's modulus and the Pauli basis keeps the trace: a
+    constant that is further off than rounding runs the general passes, which
+    apply it as it is (complex64: than 1e-12)."""
+    scale = 1.0 + off
+
+    class Scaled(jq.Operation):
+        _matrix = scale * np.array([[1, 1], [1, -1]], dtype=np.complex128) / np.sqrt(2)
+        _num_wires = 1
+        is_unitary = True
+
+    def pure():
+        for l in range(3):
+            for w in range(9):
+                jq.RX(0.1, wires=w)
+                Scaled(wires=w)
+                jq.CX(wires=[w, (w + 1) % 9])
+
+    def noisy():
+        for l in range(3):
+            for w in range(6):
+                jq.RX(0.1, wires=w)
+                jq.QubitChannel([scale * np.sqrt(0.9) * np.eye(2), scale * np.sqrt(0.1) * np.diag([1.0, -1.0])], wires=w)
+                jq.CX(wires=[w, (w + 1) % 6])
+
+    z = [jq.PauliZ(0)]
+    for circuit, n in ((pure, 9), (noisy, 6)):
+        assert _own(circuit, n, z, torch.complex128) == (off < 1e-15)
+        assert _own(circuit, n, z, torch.complex64) == (off < 1e-12)
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+def test_computed_constants_count_as_exact(dtype):
+    """Random channels of the library and Kraus sets from QR factors."""
+    rng = np.random.default_rng(7)
+
+    def noisy():
+        for _ in range(40):
+            for w in range(6):
+                jq.RX(0.1, wires=w)
+                p = rng.uniform(0, 0.3)
+                jq.DepolarizingChannel(p, wires=w)
+                jq.AmplitudeDamping(p, wires=w)
+                jq.ThermalRelaxationError(rng.uniform(0, 0.5), rng.uniform(1, 5), rng.uniform(0.5, 2), rng.uniform(0, 2), wires=w)
+                q, _ = np.linalg.qr(rng.normal(size=(4, 2)) + 1j * rng.normal(size=(4, 2)))
+                jq.QubitChannel([q[:2], q[2:]], wires=w)
+                jq.CX(wires=[w, (w + 1) % 6])
+
+    assert _own(noisy, 6, [jq.PauliZ(0)], dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+def test_circuits_and_sizes_outside_the_rules(dtype):
+    def ring(n, extra=None, noise=False):
+        def circuit():
+            for l in range(3):
+                for w in range(n):
+                    jq.Rot(0.1, 0.2, 0.3 + l, wires=w)
+                    if noise:
+                        jq.DepolarizingChannel(0.1, wires=w)
+                for w in range(n):
+                    jq.CX(wires=[w, (w + 1) % n])
+                if extra:
+                    extra()
+                    jq.RX(0.2, wires=0)
+
+        return circuit
+
+    z = [jq.PauliZ(0), jq.build_parity_observable([1, 3])]
+    assert _own(ring(9), 9, z, dtype) and not _own(ring(8), 8, z, dtype)
+    assert _own(ring(5, noise=True), 5, z, dtype) and not _own(ring(4, noise=True), 4, z, dtype)
+    for extra in (lambda: jq.CRX(0.3, wires=[0, 2]), lambda: jq.CZ(wires=[0, 1]), lambda: jq.RZZ(0.3, wires=[1, 2]),
+                  lambda: jq.CCX(wires=[0, 1, 2])):
+        assert not _own(ring(9, extra), 9, z, dtype)
+        assert not _own(ring(5, extra, True), 5, z, dtype)
+    assert not _own(ring(9), 9, [jq.PauliX(0)], dtype)
+    dense = jq.Hermitian(np.array([[1, 0.5], [0.5, 2.0]]), wires=[1], record=False)
+    assert not _own(ring(9), 9, [dense], dtype) and not _own(ring(5, noise=True), 5, [dense], dtype)
+    assert _own(ring(5, noise=True), 5, [jq.PauliX(0), jq.PauliY(3)], dtype)
+    for tune in ({"jit": -1}, {"tile_bits": 10}, {"threads": 256}):
+        assert not _own(ring(9), 9, z, dtype, tune) and not _own(ring(5, noise=True), 5, z, dtype, tune)
