@@ -148,25 +148,29 @@ typedef struct jq_tune {
                             and not run; the state buffers then hold the
                             state before them (jq_sweep applies the passes
                             the plan keeps), and other out types fail with
-                            JQ_EINVAL.  2: as 1, and what the state buffers
-                            hold is the plan's own affair, to be passed on to
-                            jq_adjoint / jq_sweep of the same plan only.  A
-                            plan of one-wire unitaries and affine permutations
+                            JQ_EINVAL.  2: as 1, and what jq_forward leaves in
+                            the state buffers for JQ_OUT_EXPVAL is the plan's
+                            own affair: it goes to jq_adjoint of the same plan
+                            with JQ_OUT_EXPVAL and nowhere else, and jq_adjoint
+                            takes no other buffer for that out type.  A plan
+                            of one-wire unitaries and affine permutations
                             (default tile sizes, jit 0, 9 qubits or more) then
-                            moves no amplitude for any permutation: its
+                            moves no amplitude for any permutation, unless the
+                            planner finds the ordinary passes cheaper: its
                             buffers hold the amplitudes at linearly mapped
                             indices, up to signs.  A density plan of one-qubit
                             gates, one-qubit channels and X / CX / SWAP-like
                             permutations with Pauli words (default tuning, 5
                             qubits or more) runs expectation values from
                             |0..0> (init NULL) on Pauli coefficients.  Calls
-                            for another out type (where nothing was absorbed)
-                            and jq_backward of a statevector plan run the
-                            circuit itself, on amplitudes at their own
-                            indices.                                           */
+                            for another out type (where nothing was absorbed),
+                            jq_sweep, and jq_backward of a statevector plan or
+                            with grad_init run the circuit itself, on entries
+                            at their own indices.                              */
 } jq_tune;
 
-/* Plan summary. */
+/* Plan summary.  Under jq_tune.expval_only = 2 the passes, stages and tile bits are
+ * those of the calls that run in the plan's own representation. */
 typedef struct jq_plan_info {
   int32_t n_qubits;
   int32_t n_bits;          /* qubits (statevector) or 2 x qubits (density)   */
@@ -245,7 +249,10 @@ JQ_API int jq_forward(const jq_plan* plan, int batch, const double* angles,
 
 /* Forward gate sweep of a statevector / density plan applied in place to a
  * resident state (no initialisation, no measurement): the state after
- * jq_sweep equals simulate_pure's result for `state` as initial state.
+ * jq_sweep equals simulate_pure's result for `state` as initial state, so that
+ * sweeps can follow one another.  `state` holds amplitudes (matrix entries) at
+ * their own indices, which a buffer that jq_forward left for JQ_OUT_EXPVAL under
+ * jq_tune.expval_only = 2 does not.
  * Replaces jaqsi/simulation.py:400-409 (_run) for a caller that keeps the
  * state on the device between circuit segments. */
 JQ_API int jq_sweep(const jq_plan* plan, int batch, const double* angles,

@@ -2514,8 +2514,7 @@ int sweep_impl(const jq_plan* plan, int batch, const double* angles, const void*
                size_t ws_bytes, cudaStream_t st) {
   using C = typename CplxT<R>::T;
   const DeviceTables* T = nullptr;
-  const bool frame = plan->frame.on;  // such a plan's buffers are its own
-  int rc = device_tables(plan, &T, !frame, st);
+  int rc = device_tables(plan, &T, true, st);  // amplitudes at their own indices, also of a frame plan
   if (rc) return rc;
   if ((rc = set_smem_attrs<R>())) return rc;
   WsLayout L = layout(plan, batch, 0);
@@ -2526,10 +2525,6 @@ int sweep_impl(const jq_plan* plan, int batch, const double* angles, const void*
   char* w = static_cast<char*>(ws);
   C* bmat = reinterpret_cast<C*>(w + L.bmat);
   double2* scratch = reinterpret_cast<double2*>(w + L.scratch);
-  if (frame) {
-    rc = frame_prep(plan, T->frame, T->blocks, T->prims, T->ops, T->const_pool, batch, angles, bmat, ZeroFill(), st);
-    return rc ? rc : frame_forward(plan, T->frame, state, batch, bmat, false, sm_count(), st);
-  }
   if ((rc = prep<R>(plan, T, batch, angles, mats, bmat, scratch, st))) return rc;
   return run_passes<R>(plan, plan->fwd, T->fwd_ops, T->fwd_steps, T->fwd_rops, T, static_cast<C*>(state), batch, bmat, 0,
                        plan->fwd.passes.size(), st, static_cast<const JitModule*>(T->jit));

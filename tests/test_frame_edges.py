@@ -14,6 +14,8 @@ import jaqsi_b200 as jq
 from jaqsi_b200 import _lib as L
 from jaqsi_b200 import simulation as sim
 from jaqsi_b200 import workloads as wl
+from oracle import sim_np as O
+from tests.helpers import to_records
 
 pytestmark = pytest.mark.gpu
 TOL = {torch.complex64: 1e-5, torch.complex128: 1e-10}
@@ -157,3 +159,59 @@ def test_reverse_call_takes_less_where_memory_is_short(monkeypatch):
         grads.append(p.grad)
     assert len(given) == 2 and given[1] < given[0]
     torch.testing.assert_close(grads[0], grads[1], atol=1e-13, rtol=0)
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("n", [9, 13])
+def test_sweeps_of_a_frame_plan_follow_one_another(n, dtype):
+    """jq_sweep applies the circuit to amplitudes at their own indices, also under
+    expval_only = 2: twice from a random state, against the oracle."""
+    rng = np.random.default_rng(n)
+
+    def circuit(p):
+        for l in range(2):
+            for w in range(n):
+                jq.Rot(p[l, w, 0], p[l, w, 1], p[l, w, 2], wires=w)
+            if l == 0:
+                for w in range(n):
+                    jq.CX(wires=[w, (w + 1) % n])
+                jq.PauliX(wires=2)
+                jq.SWAP(wires=[0, n - 1])
+
+    base = torch.tensor(rng.uniform(0, 2 * np.pi, (2, n, 3)))
+    script = jq.Script(circuit, n_qubits=n)
+    plan = sim.get_plan(sim.lower_tape(script.record(base), n), *sim._lower_obs([jq.PauliZ(0)], n), n,
+                        L.JQ_STATEVECTOR, dtype)
+    psi = rng.normal(size=2**n) + 1j * rng.normal(size=2**n)
+    psi /= np.linalg.norm(psi)
+    angles = base.reshape(-1).to("cuda")
+    state = torch.tensor(psi, dtype=dtype, device="cuda")
+    ws = torch.empty(plan.workspace_bytes(1), dtype=torch.uint8, device="cuda")
+    recs = to_records(script.record(base))
+    for _ in range(2):
+        L.check(plan._lib.jq_sweep(plan.handle, 1, sim._ptr(angles), None, sim._ptr(state), sim._ptr(ws), ws.numel(),
+                                   sim._stream()))
+        psi = O.simulate_pure(recs, n, psi)
+        np.testing.assert_allclose(state.cpu().numpy(), psi, atol=TOL[dtype], rtol=0)
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+def test_sweeps_of_a_pauli_plan_work_on_matrix_entries(dtype):
+    n, layers = 5, 2
+    rng = np.random.default_rng(3)
+    obs = [jq.PauliZ(0)]
+    general, own = _noisy_plans(n, layers, 0.02, obs, dtype)
+    angles = torch.tensor(rng.uniform(0, 2 * np.pi, own.n_angles), device="cuda")
+    a = rng.normal(size=(2**n, 2**n)) + 1j * rng.normal(size=(2**n, 2**n))
+    rho = a @ a.conj().T
+    rho = torch.tensor(rho / np.trace(rho), dtype=dtype, device="cuda")
+    got = []
+    for plan in (general, own):
+        state = rho.clone()
+        ws = torch.empty(plan.workspace_bytes(1), dtype=torch.uint8, device="cuda")
+        for _ in range(2):
+            L.check(plan._lib.jq_sweep(plan.handle, 1, sim._ptr(angles), None, sim._ptr(state), sim._ptr(ws), ws.numel(),
+                                       sim._stream()))
+        got.append(state.cpu().numpy())
+    np.testing.assert_allclose(got[1], got[0], atol=TOL[dtype], rtol=0)
+    assert abs(np.trace(got[1]) - 1) < 10 * TOL[dtype]
