@@ -15,7 +15,7 @@ from jaqsi_b200 import _lib as L
 from jaqsi_b200 import simulation as sim
 from jaqsi_b200 import workloads as wl
 from oracle import sim_np as O
-from tests.helpers import to_records
+from tests.helpers import obs_records, to_records
 
 pytestmark = pytest.mark.gpu
 TOL = {torch.complex64: 1e-5, torch.complex128: 1e-10}
@@ -215,3 +215,65 @@ def test_sweeps_of_a_pauli_plan_work_on_matrix_entries(dtype):
         got.append(state.cpu().numpy())
     np.testing.assert_allclose(got[1], got[0], atol=TOL[dtype], rtol=0)
     assert abs(np.trace(got[1]) - 1) < 10 * TOL[dtype]
+
+
+def _values_and_gradients(plan, angles, rows):
+    """Expectation values and the gradients of their weighted sum, `rows` instances a call."""
+    values, grads = [], []
+    for a in angles.split(rows):
+        state, out = sim._forward_launch(plan, L.JQ_OUT_EXPVAL, a.shape[0], 0, a, None, None)
+        ct = torch.linspace(0.5, 1.5, plan.n_obs, dtype=torch.float64, device="cuda").expand(a.shape[0], -1)
+        values.append(out)
+        grads.append(sim._grad_launch(plan, L.JQ_OUT_EXPVAL, a.shape[0], 0, (True, False, False), a, None, None, state, ct)[0])
+    return torch.cat(values), torch.cat(grads)
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("n,batch,noisy", [(9, 6000, False), (10, 5000, False), (12, 1300, False), (13, 600, False),
+                                           (16, 80, False), (5, 5000, True), (6, 1300, True), (8, 80, True)])
+def test_batches_of_more_tiles_than_fit_at_once(n, batch, noisy, dtype):
+    """A CTA goes from one instance's tiles to the next one's: new gate tables, sums
+    handed over.  Every instance has angles of its own; a call on eight of them
+    has a CTA a tile.  The kernels do the same arithmetic on a tile in both, so
+    that only the order of float64 additions differs."""
+    layers = 2
+    with jq.recording() as tape:
+        if noisy:
+            wl.noisy_ansatz(n, layers, np.zeros((layers, n, 3)), 0.01, 0.02)
+        else:
+            wl.rot_ring(n, layers, np.zeros((layers, n, 3)))
+    lw = sim.lower_tape(tape, n)
+    obs = [jq.PauliZ(w) for w in range(n)]
+    specs, _ = sim._lower_obs(obs, n)
+    statics = [st[:10] + (1,) + st[11:] if st[3] >= 0 else st for st in lw.statics]  # every angle trainable
+    mode = L.JQ_DENSITY if noisy else L.JQ_STATEVECTOR
+    general, plan = [sim.Plan(statics, specs, n, mode, dtype, {"expval_only": e}) for e in (1, 2)]
+    assert plan.info != general.info
+    bits = 2 * n if noisy else n
+    tile = bits if bits <= 10 or (bits == 12 and not noisy) else 11
+    most = torch.cuda.get_device_properties(0).multi_processor_count * min(32, 2048 // (1 << (tile - 4)))
+    assert batch << (bits - tile) > most
+    angles = torch.tensor(np.random.default_rng(n).uniform(0, 2 * np.pi, (batch, plan.n_angles)), device="cuda")
+    for all_at_once, few in zip(_values_and_gradients(plan, angles, batch), _values_and_gradients(plan, angles, 8)):
+        torch.testing.assert_close(all_at_once, few, atol=1e-12, rtol=0)
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("n,layers", [(9, 5), (10, 7), (11, 9), (12, 5), (12, 12)])
+def test_whole_state_tiles_of_many_stages(n, layers, dtype):
+    """States of one tile: more stages than tile flips are kept for, and (the longest)
+    more than a pass holds, against the oracle."""
+    rng = np.random.default_rng(n * layers)
+    base = rng.uniform(0, 2 * np.pi, (layers, n, 3))
+    script = jq.Script(lambda a: wl.rot_ring(n, layers, a), n_qubits=n)
+    obs = [jq.PauliZ(0), jq.build_parity_observable([1, n - 1])]
+    lw = sim.lower_tape(script.record(torch.tensor(base)), n)
+    info = sim.get_plan(lw, *sim._lower_obs(obs, n), n, L.JQ_STATEVECTOR, dtype).info
+    assert info["n_stages_fwd"] > 8 and info["n_tile_ops_fwd"] == n * layers
+    assert info["n_passes_fwd"] == (1 if info["n_stages_fwd"] <= 24 else 2)
+    params = torch.tensor(base, requires_grad=True)
+    ev = script.execute("expval", obs, args=(params,), dtype=dtype)
+    ev.sum().backward()
+    want, grad = O.adjoint_grad(to_records(script.record(torch.tensor(base))), n, obs_records(obs), ct=np.ones(2))
+    np.testing.assert_allclose(ev.detach().cpu().numpy(), want, atol=TOL[dtype], rtol=0)
+    np.testing.assert_allclose(params.grad.numpy().reshape(-1), grad, atol=TOL[dtype] * 2, rtol=0)
