@@ -638,7 +638,10 @@ _Execute.forward.__signature__ = inspect.signature(_Execute.forward)
 def _plain(tensors) -> bool:
     """Whether a call on these tensors needs no autograd Function: nothing to
     record (gradients off or not asked for), no torch.func transform around
-    any of them and no forward-mode level open."""
+    any of them, no forward-mode level open and no torch.jit.trace running, which
+    records the Function and would keep the bare call's output as a constant."""
+    if torch._C._get_tracing_state() is not None:
+        return False
     grad = torch.is_grad_enabled()
     for t in tensors:
         if t is not None and ((grad and t.requires_grad) or _functorch_wrapped(t)):

@@ -81,3 +81,28 @@ def test_indices_outlive_a_dropped_trace_while_another_stream_reads_them():
     assert busy, "the second stream finished too early to tell"
     assert read[0] not in [t.data_ptr() for t in taken]
     torch.cuda.synchronize()
+
+
+@pytest.mark.gpu
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("noisy", [False, True])
+def test_traced_calls_run_the_circuit(noisy):
+    """torch.jit.trace records the call as an autograd Function: the traced module
+    runs it on other inputs."""
+
+    def circuit(p):
+        for w in range(2):
+            jq.RY(p[w], wires=w)
+            if noisy:
+                jq.DepolarizingChannel(0.1, wires=w)
+
+    script = jq.Script(circuit, n_qubits=2)
+    obs = [jq.PauliZ(0), jq.PauliZ(1)]
+    x = torch.tensor([0.3, 0.4], dtype=torch.float64, device="cuda")
+
+    def call(p):
+        return script.execute("expval", obs, args=(p,))
+
+    want = call(x + 1)
+    traced = torch.jit.trace(call, (x,), check_trace=False)
+    assert torch.equal(traced(x + 1), want) and torch.equal(traced(x), call(x))
