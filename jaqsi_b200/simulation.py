@@ -637,10 +637,11 @@ _Execute.forward.__signature__ = inspect.signature(_Execute.forward)
 
 def _plain(tensors) -> bool:
     """Whether a call on these tensors needs no autograd Function: nothing to
-    record (gradients off or not asked for), no torch.func transform around
-    any of them, no forward-mode level open and no torch.jit.trace running, which
-    records the Function and would keep the bare call's output as a constant."""
-    if torch._C._get_tracing_state() is not None:
+    record (gradients off or not asked for), no torch.func transform open (inside
+    one even a new buffer is a wrapper without memory), no forward-mode level open
+    and no torch.jit.trace running, which records the Function and would keep the
+    bare call's output as a constant."""
+    if torch._C._get_tracing_state() is not None or torch._C._are_functorch_transforms_active():
         return False
     grad = torch.is_grad_enabled()
     for t in tensors:

@@ -106,3 +106,28 @@ def test_traced_calls_run_the_circuit(noisy):
     want = call(x + 1)
     traced = torch.jit.trace(call, (x,), check_trace=False)
     assert torch.equal(traced(x + 1), want) and torch.equal(traced(x), call(x))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("noisy", [False, True])
+def test_circuits_without_parameters_inside_torch_func(noisy):
+    """Inside a transform buffers are wrappers: a circuit that takes nothing from it
+    still runs."""
+
+    def circuit(*p):
+        jq.H(wires=0)
+        jq.CX(wires=[0, 1])
+        if noisy:
+            jq.DepolarizingChannel(0.3, wires=1)
+
+    script = jq.Script(circuit, n_qubits=2)
+    obs = [jq.build_parity_observable([0, 1])]
+    value = script.execute("expval", obs)
+    x = torch.tensor([2.0, 3.0], dtype=torch.float64, device="cuda")
+
+    def f(y):
+        return (y * y * script.execute("expval", obs)).sum()
+
+    assert torch.allclose(torch.func.grad(f)(x), 2 * x * value)
+    assert torch.allclose(torch.func.jvp(f, (x,), (torch.ones_like(x),))[1], (2 * x * value).sum())
+    assert torch.allclose(torch.func.vmap(lambda y: y * script.execute("expval", obs)[0])(x), x * value)
