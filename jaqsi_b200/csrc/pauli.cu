@@ -590,14 +590,21 @@ __global__ void k_pauli_expval(const F* __restrict__ s, int nb, const PauliObs* 
 }
 template <typename F>
 __global__ void k_pauli_seed(F* __restrict__ lam, int nb, const PauliObs* __restrict__ obs, int n_obs, int batch,
-                             const double* __restrict__ ct) {
+                             const double* __restrict__ ct, double* __restrict__ gacc, int64_t gstride) {
   const int64_t inst = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (inst >= batch) return;
   // one thread an instance: words may coincide
+  bool finite = true;
   for (int o = 0; o < n_obs; ++o) {
     F* p = lam + (inst << nb) + obs[o].index;
-    *p = static_cast<F>(static_cast<double>(*p) + obs[o].coeff * ct[inst * n_obs + o]);
+    const double w = obs[o].coeff * ct[inst * n_obs + o];
+    finite = finite && isfinite(w);
+    *p = static_cast<F>(static_cast<double>(*p) + w);
   }
+  // a cotangent that is not finite leaves no entry of lambda's matrix finite, and
+  // so no gradient of the instance, also where its word does not reach a gate
+  if (!finite && gacc)
+    for (int64_t i = 0; i < gstride; ++i) gacc[inst * gstride + i] = __longlong_as_double(0x7ff8000000000000LL);
 }
 
 template <typename F, int T> constexpr int fwd_ctas() { return sizeof(F) == 4 ? (T == 11 ? 8 : 16) : (T == 11 ? 5 : 10); }
@@ -724,12 +731,12 @@ int backward_t(const jq_plan* plan, const FrameDev& d, const DeviceTables& T, in
           return rc;
   JQ_CUDA(cudaMemsetAsync(lam, 0, bytes, st));
   const int no = static_cast<int>(plan->pauli_obs.size());
-  k_pauli_seed<F><<<blocks_for(batch, 64), 64, 0, st>>>(lam, plan->n_bits, static_cast<const PauliObs*>(T.pauli_obs), no,
-                                                        batch, ct);
-  JQ_CUDA(cudaGetLastError());
   const int64_t gstride = 12 * static_cast<int64_t>(fp.n_grad);
   const bool want = grad && fp.n_grad > 0;
   if (want) JQ_CUDA(cudaMemsetAsync(gacc, 0, sizeof(double) * gstride * batch, st));
+  k_pauli_seed<F><<<blocks_for(batch, 64), 64, 0, st>>>(lam, plan->n_bits, static_cast<const PauliObs*>(T.pauli_obs), no,
+                                                        batch, ct, want ? gacc : nullptr, gstride);
+  JQ_CUDA(cudaGetLastError());
   for (int64_t c = std::max<int64_t>(nck, 1) - 1; c >= 0; --c) {
     const int64_t p0 = c * S, p1 = std::min(P, p0 + S);
     auto input = [&](int64_t p) { return nck > 0 ? (p == p0 ? slot(c) : seg(p - p0 - 1)) : slot(p); };

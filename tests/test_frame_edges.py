@@ -46,6 +46,28 @@ def test_noisy_values_of_an_angle_that_is_not_finite(n, bad, gate, dtype):
     assert torch.equal(ev[0], ev[2])
 
 
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("n", [5, 6])
+def test_noisy_gradients_of_a_cotangent_that_is_not_finite(n, bad, dtype):
+    """Every gradient of that sample is NaN, also of gates the observable's word does
+    not reach; those of the others are not."""
+
+    def circuit(p):
+        for w in range(n):
+            jq.RY(p[w], wires=w)
+            jq.DepolarizingChannel(0.1, wires=w)
+
+    params = torch.full((3, n), 0.3, dtype=torch.float64, requires_grad=True)
+    script = jq.Script(circuit, n_qubits=n)
+    ev = script.execute("expval", [jq.PauliZ(w) for w in range(n)], args=(params,), in_axes=(0,), dtype=dtype)
+    ct = torch.ones_like(ev)
+    ct[1, 2] = bad
+    ev.backward(ct)
+    assert torch.isnan(params.grad[1]).all()
+    assert torch.isfinite(params.grad[[0, 2]]).all() and torch.equal(params.grad[0], params.grad[2])
+
+
 @pytest.mark.parametrize("n", [9, 10, 11, 12, 13, 15])
 def test_frame_cotangent_sums_of_small_states_are_float64(n):
     """Complex64 states below 2^16 amplitudes.  Wire a starts in |+> and has no gate,
