@@ -28,7 +28,7 @@ struct PassArg {
   uint32_t g[kFrameMaxT];
   uint32_t cs[kFrameMaxT];
   uint32_t opos[32];
-  int32_t nb, nouter, c;
+  int32_t nb, nouter;
   int32_t st0, nst;
   int32_t direct;
 };
@@ -146,7 +146,6 @@ PassArg pass_arg(const FramePass& p, int nb, bool adjoint) {
   std::memcpy(a.opos, p.opos, sizeof(a.opos));
   a.nb = nb;
   a.nouter = p.nouter;
-  a.c = p.c;
   a.st0 = p.st0;
   a.nst = p.nst;
   a.direct = adjoint ? p.adirect : p.direct;

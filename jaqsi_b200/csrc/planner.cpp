@@ -988,10 +988,13 @@ int build_plan(const jq_op* ops, int n_ops, const jq_obs* obs, int n_obs, int n_
     // States of up to 12 bits are one tile.  Larger ones take tiles of 11 bits:
     // at 24 qubits complex64 10, 11 and 12 bits measured 3.62, 3.63 and 3.81 ms,
     // at 20 qubits (forward + adjoint) 3.98, 3.63 and 3.62 ms; with passes launched
-    // ahead 3.17, 3.10, 3.29 and 2.89, 2.69, 2.81 ms.  Runs of 64 bytes
-    // (3 low bits) leave more of a tile to the masks; beyond the L2 (126 MB) runs of
-    // 128 bytes are faster in spite of more passes: 24 qubits 3.51 against 3.63 ms,
-    // 20 qubits 3.87 against 3.63 ms.
+    // ahead 3.17, 3.10, 3.29 and 2.89, 2.69, 2.81 ms.  Runs of 64 bytes in complex64
+    // (3 low bits) leave more of a tile to the masks; a complex64 state beyond the L2
+    // (126 MB) takes runs of 128 bytes.  2 / 3 / 4 low bits, forward: 24 qubits x 20
+    // layers complex64 3.54 / 3.08 / 3.05 ms (30, 34, 40 passes), complex128 6.10 / 5.84
+    // / 5.99; forward + adjoint, growing ranges, 24 qubits x 10 layers complex64 9.3 /
+    // 7.1 / 6.6, 20 qubits x 50 layers 2.84 / 2.59 / 2.60 (94, 108, 124 passes), x 20
+    // layers complex128 1.83 / 1.65 / 1.83; 16 qubits complex128 0.215 / 0.221 / 0.221.
     const int ft = nb <= kFrameMaxT ? nb : 11;
     const int fc = dtype == JQ_C64 && nb >= 24 ? 4 : 3;
     FramePlan frame;

@@ -299,3 +299,86 @@ def test_whole_state_tiles_of_many_stages(n, layers, dtype):
     want, grad = O.adjoint_grad(to_records(script.record(torch.tensor(base))), n, obs_records(obs), ct=np.ones(2))
     np.testing.assert_allclose(ev.detach().cpu().numpy(), want, atol=TOL[dtype], rtol=0)
     np.testing.assert_allclose(params.grad.numpy().reshape(-1), grad, atol=TOL[dtype] * 2, rtol=0)
+
+
+def _linear(rng, k):
+    """A random invertible 0/1 matrix over GF(2) as columns, and its permutation."""
+    while True:
+        col = [int(v) for v in rng.integers(1, 1 << k, k)]
+        to = [0] * (1 << k)
+        for x in range(1 << k):
+            for i in range(k):
+                if x >> i & 1:
+                    to[x] ^= col[i]
+        if len(set(to)) == 1 << k:
+            return to
+
+
+def _permuting(rng, k, shift):
+    """A gate that takes basis state x to A x ^ b (b = 0 unless `shift`)."""
+    to = _linear(rng, k)
+    b = int(rng.integers(1 << k)) if shift else 0
+    perm = [0] * (1 << k)
+    for x, y in enumerate(to):
+        perm[y ^ b] = x  # output row r takes input column perm[r]
+    m = np.zeros((1 << k, 1 << k), dtype=np.complex128)
+    m[np.arange(1 << k), perm] = 1
+    return type(f"Perm{k}_{rng.integers(1 << 40)}", (jq.Operation,),
+                {"_matrix": m, "_num_wires": k, "is_unitary": True, "_structure": jq.operations.GateStructure(permutation=tuple(perm))})
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("n,noisy", [(9, False), (12, False), (13, False), (16, False), (5, True), (6, True), (7, True), (8, True)])
+def test_every_permutation_that_is_accepted(n, noisy, dtype):
+    """Random affine permutations of two to six wires (linear ones of two to four
+    on Pauli words) in any wire order, rotations by every generator, constants and
+    random Kraus sets, Pauli words with either sign: against the general passes."""
+    rng = np.random.default_rng(31 * n + noisy)
+
+    def circuit(p):
+        k = 0
+        for _ in range(4):
+            for w in range(n):
+                kind = int(rng.integers(6))
+                if kind == 0:
+                    jq.Rot(p[k], p[k + 1], p[k + 2], wires=w)
+                    k += 3
+                elif kind < 4:
+                    jq.PauliRot(p[k], "XYZ"[kind - 1], wires=[w])
+                    k += 1
+                elif kind == 4:
+                    jq.H(wires=w)
+                    jq.S(wires=w)
+                if noisy and rng.integers(2):
+                    q, _ = np.linalg.qr(rng.normal(size=(6, 2)) + 1j * rng.normal(size=(6, 2)))
+                    jq.QubitChannel([np.sqrt(0.9) * np.eye(2)] + [np.sqrt(0.1) * q[2 * i:2 * i + 2] for i in range(3)], wires=w)
+            for _ in range(3):
+                size = int(rng.integers(2, 5 if noisy else 7))
+                wires = [int(w) for w in rng.choice(n, size, replace=False)]
+                _permuting(rng, size, not noisy)(wires=wires)
+        for w in range(n):
+            jq.RY(p[k + w], wires=w)
+        return k + n
+
+    with jq.recording() as tape:
+        count = circuit(torch.zeros(16 * n + 16))
+    assert count <= 16 * n + 16
+    pauli = [np.eye(2), np.array([[0, 1], [1, 0]]), np.array([[0, -1j], [1j, 0]]), np.diag([1.0, -1.0])]
+    obs = []
+    for _ in range(12):
+        wires = [int(w) for w in rng.choice(n, 3, replace=False)]
+        m = np.array([[rng.choice([-1.5, 0.5, 2.0])]])
+        for _ in wires:
+            m = np.kron(m, pauli[int(rng.integers(4)) if noisy else 3 * int(rng.integers(2))])
+        obs.append(jq.Hermitian(m, wires=wires, record=False))
+    lw = sim.lower_tape(tape, n)
+    specs, _ = sim._lower_obs(obs, n)
+    statics = [st[:10] + (1,) + st[11:] if st[3] >= 0 else st for st in lw.statics]  # every angle trainable
+    mode = L.JQ_DENSITY if noisy else L.JQ_STATEVECTOR
+    general, own = [sim.Plan(statics, specs, n, mode, dtype, {"expval_only": e, "jit": 0 if e == 2 else -1}) for e in (1, 2)]
+    assert own.info["n_tile_ops_fwd"] != general.info["n_tile_ops_fwd"]  # permutations are none in either
+    angles = torch.tensor(rng.uniform(0, 2 * np.pi, (2, own.n_angles)), device="cuda")
+    got, want = _values_and_gradients(own, angles, 2), _values_and_gradients(general, angles, 2)
+    for g, w in zip(got, want):
+        np.testing.assert_allclose(g.cpu().numpy(), w.cpu().numpy(), atol=TOL[dtype] * 2.0 * len(obs), rtol=0)
+    assert got[0].abs().max() > 1e-3 and got[1].abs().max() > 1e-3

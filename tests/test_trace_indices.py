@@ -1,5 +1,6 @@
-"""The index tensors a cached trace keeps: usable by every later call, whatever
-was open around the first one, on any stream."""
+"""What a call keeps and skips on the host: the index tensors of a cached trace
+(usable by every later call, whatever was open around the first one, on any
+stream), and the autograd Function (not inside torch.jit.trace and torch.func)."""
 import pytest
 import torch
 
