@@ -212,18 +212,27 @@ bool pauli_map(const std::vector<cd>& s, double tol) {
 }
 
 // Whether a frame plan costs no more than the specialised passes, of which a stage
-// holds gates that need not commute.  In units of a general gate a frame stage
-// costs the same below 20 qubits (both are latency) and 2.5 gates from there on, a
-// pass 2 in either, a call 4 more without the frame (its start state is written and
-// read).  Measured forward, general / frame (us): 24 qubits complex64, 12 layers on
-// two wires (24 gates, 12 stages) 224 / 315, on three (36, 12) 323 / 315, ring of 4
-// layers (96, 27) 830 / 633; one gate a stage 224 / 514 (24), 81 / 160 (22), 40 / 64
-// (20), 33 / 38 (16); complex128 two wires 365 / 535 (24), 50 / 57 (20), 35 / 32 (16).
+// holds gates that need not commute.  In units of a general gate a pass costs 2 in
+// either and a call 4 more without the frame (its start state is written and read);
+// a frame stage costs little more than one gate while a pass is the latency of its
+// tiles, and 2.5 from about 2^19 amplitudes on, where it is their throughput.
+// Measured on one B200, general / frame (us), forward and forward + adjoint:
+//   24 qubits complex64: ring of 4 layers (96 gates, 27 stages) 830 / 633, 4072 / 2235;
+//     12 layers on three wires (36, 12) 323 / 315, 1904 / 1067, on two (24, 12)
+//     224 / 315, 1338 / 1065, one gate a stage (24, 24) 224 / 514, 1336 / 1841;
+//     a staircase of 12 layers, CX between rotations (288, 215) 2367 / 4106, 12.5 / 15.3 ms
+//   24 qubits complex128: the staircase 4.1 / 7.9, 19.3 / 30.7 ms, two wires 365 / 535, 1829 / 1985
+//   20 qubits complex64: staircase of 4 layers (80, 50) 104 / 119, 379 / 349
+//   19 qubits: of 12 layers (228, 155) complex64 242 / 281, 703 / 897, complex128 271 / 374,
+//     878 / 1054, two wires 33 / 34, 102 / 86 and 38 / 42, 121 / 117
+//   18 qubits: of 12 layers (216, 135) 214 / 142, 645 / 519 and 252 / 273, 765 / 822
+//   16 qubits: of 4 layers (64, 19) 74 / 34, 210 / 86, one gate a stage 33 / 38, 98 / 96
 // Below 2^16 amplitudes the alternative is an interpreter: one gate a stage 45 / 44 at
 // 12 qubits complex64 and 54 / 56 in complex128, everything else is further apart.
-bool frame_pays(const FramePlan& f, size_t general_passes, int nb) {
+bool frame_pays(const FramePlan& f, size_t general_passes, int nb, int dtype) {
   if (nb < 16) return true;
-  const double stage = nb >= 20 ? 2.5 : 1.0;
+  const bool c64 = dtype == JQ_C64;
+  const double stage = nb >= 20 ? (c64 ? 2.5 : 2.75) : nb == 19 ? (c64 ? 2.0 : 2.5) : nb == 18 && !c64 ? 1.75 : 1.25;
   return stage * static_cast<double>(f.stages.size()) + 2.0 * static_cast<double>(f.passes.size()) <=
          static_cast<double>(f.gates.size()) + 2.0 * static_cast<double>(general_passes) + 4.0;
 }
@@ -999,7 +1008,7 @@ int build_plan(const jq_op* ops, int n_ops, const jq_obs* obs, int n_obs, int n_
     const int fc = dtype == JQ_C64 && nb >= 24 ? 4 : 3;
     FramePlan frame;
     if (ok && frame_schedule(fops, nb, ft, fc, dtype == JQ_C64 ? 8 : 16, ft == nb ? kFrameMaxStages : kFrameBallot, &zt, &zsign, &frame) &&
-        (!plan->jit || frame_pays(frame, plan->fwd.passes.size(), nb))) {
+        (!plan->jit || frame_pays(frame, plan->fwd.passes.size(), nb, dtype))) {
       plan->frame = std::move(frame);
       plan->frame_obs = plan->obs;
       for (int i = 0; i < n_obs; ++i) {

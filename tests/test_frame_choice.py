@@ -65,6 +65,30 @@ def test_deep_circuits_on_few_wires_keep_the_specialised_passes(dtype):
     assert _own(_serial(12, 50), 12, z, dtype) and _own(_wires(15, 50, 2), 15, z, dtype)
 
 
+def _staircase(n, layers):
+    """A CX after every rotation: each gate waits for the one on the wire before."""
+
+    def circuit():
+        for l in range(layers):
+            for w in range(n):
+                jq.Rot(0.1, 0.2 + l, 0.3, wires=w)
+                if w + 1 < n:
+                    jq.CX(wires=[w, w + 1])
+
+    return circuit
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+def test_staircases_run_in_the_frame_up_to_18_qubits(dtype):
+    z = [jq.PauliZ(0)]
+    for n in (9, 12, 14, 16, 17):
+        assert _own(_staircase(n, 4), n, z, dtype), n
+    assert _own(_staircase(18, 12), 18, z, torch.complex64)
+    for n in (19, 20, 22, 24):
+        assert not _own(_staircase(n, 12), n, z, dtype), n
+        assert not _own(_staircase(n, 4), n, z, dtype), n
+
+
 @pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
 @pytest.mark.parametrize("family", [wl.sweep_ansatz, wl.strongly_entangling, wl.rot_ring])
 def test_circuits_on_every_wire_run_in_the_frame(family, dtype):
