@@ -382,3 +382,79 @@ def test_every_permutation_that_is_accepted(n, noisy, dtype):
     for g, w in zip(got, want):
         np.testing.assert_allclose(g.cpu().numpy(), w.cpu().numpy(), atol=TOL[dtype] * 2.0 * len(obs), rtol=0)
     assert got[0].abs().max() > 1e-3 and got[1].abs().max() > 1e-3
+
+
+@pytest.mark.parametrize("n,noisy", [(9, False), (13, False), (5, True), (6, True)])
+def test_torch_func_transforms_in_both_representations(n, noisy):
+    """jacrev, jvp, vmap and a batched initial state through the plan's own state
+    buffers, against one reverse call per value."""
+    layers = 2
+    body = (lambda a: wl.noisy_ansatz(n, layers, a, 0.01, 0.02)) if noisy else (lambda a: wl.rot_ring(n, layers, a))
+    script = jq.Script(body, n_qubits=n)
+    obs = [jq.PauliZ(0), jq.PauliZ(n - 1), jq.build_parity_observable([1, 2])]
+    p = torch.tensor(np.random.default_rng(n).uniform(0, 2 * np.pi, (layers, n, 3)), device="cuda")
+
+    def f(x):
+        return script.execute("expval", obs, args=(x,))
+
+    rows = []
+    for o in range(len(obs)):
+        x = p.clone().requires_grad_(True)
+        rows.append(torch.autograd.grad(f(x)[o], x)[0])
+    rows = torch.stack(rows)
+    torch.testing.assert_close(torch.func.jacrev(f)(p), rows, atol=1e-12, rtol=0)
+    v = torch.randn(p.shape, generator=torch.Generator("cuda").manual_seed(1), device="cuda", dtype=torch.float64)
+    value, tangent = torch.func.jvp(f, (p,), (v,))
+    torch.testing.assert_close(value, f(p), atol=1e-13, rtol=0)
+    torch.testing.assert_close(tangent, (rows * v).sum((1, 2, 3)), atol=1e-11, rtol=0)
+    many = torch.stack([p, p + 0.1, 2 * p])
+    each = torch.stack([f(x) for x in many])
+    torch.testing.assert_close(torch.func.vmap(f)(many), each, atol=1e-13, rtol=0)
+    torch.testing.assert_close(script.execute("expval", obs, args=(many,), in_axes=(0,)), each, atol=1e-13, rtol=0)
+    grads = torch.func.vmap(torch.func.grad(lambda x: f(x).sum()))(many)
+    torch.testing.assert_close(grads[0], rows.sum(0), atol=1e-12, rtol=0)
+
+
+@pytest.mark.parametrize("n,noisy", [(9, False), (13, False), (6, True)])
+def test_threads_on_streams_of_their_own(n, noisy):
+    """Four threads, each on its own stream, share a script and its plan from its
+    first call on: the results of calls one after the other."""
+    import threading
+
+    layers = 2
+    body = (lambda a: wl.noisy_ansatz(n, layers, a, 0.01, 0.02)) if noisy else (lambda a: wl.rot_ring(n, layers, a))
+    obs = [jq.PauliZ(0), jq.PauliZ(n - 1)]
+    params = torch.tensor(np.random.default_rng(n).uniform(0, 2 * np.pi, (4, layers, n, 3)), device="cuda")
+
+    def step(script, k):
+        x = params[k].clone().requires_grad_(True)
+        value = script.execute("expval", obs, args=(x,))
+        return value.detach(), torch.autograd.grad(value.sum(), x)[0]
+
+    shared = jq.Script(body, n_qubits=n)
+    got = [[] for _ in range(4)]
+    failed = []
+
+    def work(k, stream):
+        try:
+            with torch.cuda.stream(stream):
+                for _ in range(20):
+                    got[k].append(step(shared, k))
+        except Exception as e:  # pragma: no cover - reported below
+            failed.append(e)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(k, torch.cuda.Stream())) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed, failed
+    alone = jq.Script(body, n_qubits=n)
+    for k in range(4):
+        want = step(alone, k)
+        assert len(got[k]) == 20
+        for value, grad in got[k]:
+            torch.testing.assert_close(value, want[0], atol=1e-13, rtol=0)
+            torch.testing.assert_close(grad, want[1], atol=1e-12, rtol=0)
