@@ -174,11 +174,12 @@ __device__ __forceinline__ void pass_tables(const FrameStage* __restrict__ st, i
 // up to four gates and stores.
 //
 // Bound by instruction issue and its latencies (57% of issue slots, 89 instructions
-// an amplitude and pass of 12 gates; FMA pipe 43%, HBM 42% busy).  24 qubits, 20 layers, complex64: 40 passes of 75 us for 133
-// stages against 66 passes of 60 us for 157, 4.19 -> 3.06 ms a call (tiles copied 8
-// bytes at a time instead of 16 cost 0.27 ms).  Five CTAs an SM; six (79
-// registers) were 18% slower.  Pairs of amplitudes in packed FMAs
-// throughout: 1.5 times slower, register moves for every packed operand.
+// an amplitude and pass of 12 gates; FMA pipe 43%, HBM 42% busy).  24 qubits, 20
+// layers, complex64: 40 passes of 75 us for 133 stages against 66 passes of 60 us
+// for 157, 4.19 -> 3.06 ms a call (tiles copied 8 bytes at a time instead of 16 cost
+// 0.27 ms).  Five CTAs an SM; six (79 registers) were 18% slower.  Pairs of
+// amplitudes in packed FMAs throughout: 1.5 times slower, register moves for every
+// packed operand.
 template <typename C, int T, int MINB>
 __global__ void __launch_bounds__(1 << (T - 4), MINB)
     k_frame_fwd(C* __restrict__ state, const PassArg P, const FrameStage* __restrict__ stages,
